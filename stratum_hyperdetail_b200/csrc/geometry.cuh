@@ -182,12 +182,13 @@ SD bool featureSlabMiss(const Feat& f, Span range) { return f.shape < 0 || range
 static __device__ __noinline__ float featureAfterSlabOOL(Feat f, f3 ro, f3 rd, f3 p, f3 d, f3 inv, float cone) {
   return featureHitCore(f, ro, rd, p, d, inv, cone);
 }
+SD bool plainBox(const Feat& f) { return f.shape == 0 && !((f.material == 0 || f.material == 1) && f.h.y > 1.0f); }
+SD float plainBoxHit(Span range) {
+  float t = range.lo > 0.001f ? range.lo : range.hi;
+  return t <= 0.001f ? kFar : t;
+}
 SD float featureAfterSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, f3 inv, Span range, float cone) {
-  if (f.shape == 0 && !((f.material == 0 || f.material == 1) && f.h.y > 1.0f)) {  // plain box
-    float t = range.lo > 0.001f ? range.lo : range.hi;
-    return t <= 0.001f ? kFar : t;
-  }
-  return featureAfterSlabOOL(f, ro, rd, p, d, inv, cone);
+  return plainBox(f) ? plainBoxHit(range) : featureAfterSlabOOL(f, ro, rd, p, d, inv, cone);
 }
 
 // Surface normal of a feature at a point (geometry.cu:92-114).

@@ -10,9 +10,19 @@
 //    time: the group's records are staged in shared memory, one per lane --
 //    loaded from the table's group cache (group_cache.cuh) when it holds the
 //    group, else built by the random-access grammar (grammar_ra.cuh) and, when
-//    the cache has room, stored there for every later evaluation -- and every
-//    lane waiting on that key tests them in index order with one inlined
-//    intersection routine and its precomputed inverse directions;
+//    the cache has room, stored there for every later evaluation.  The lanes
+//    then stand for records: each tests its one or two records against all the
+//    waiting rays at once, taken as a packet (packetMayHit).  Most evaluations
+//    end here (63 % of them on the street pose, 38 % on the aerial one, keep no
+//    record; the others keep 2-5 of up to 56), and every lane waiting on the key
+//    tests the records kept, in index order, with one inlined intersection
+//    routine and its precomputed inverse directions.  What bounds the kernel is
+//    instruction issue and latency: walking the waiting rays through all the
+//    records behind one box test per run of four took 1,000 (aerial) to 2,500
+//    (street) instructions per evaluation, this takes about 250; six-view
+//    1600x900 trace 7.61 -> 6.80 ms (street 1.76 -> 1.36, aerial 3.15 -> 2.89).
+//    One lane per (ray, record) pair by ballots over every waiting ray (its own
+//    candidate mask per lane) measured 7.27 ms;
 //  * the winner's normal, material and seed are recomputed once per ray.
 //
 // Each lane's leaves are visited in the reference's order and each test sees
@@ -31,9 +41,8 @@ namespace st {
 // instruction cache (measured faster than inlining it).
 static __device__ __noinline__ Feat featureAtOOL(LotDesc L, int g, int i) { return featureAt(L, g, i); }
 
-// Sub-group culling: every run of kRun staged features gets a box (in the
-// lot frame) that contains every distance any of them can return, and a lane
-// tests a run's features only when its ray enters that box nearer than its
+// A box (in the lot frame) that contains every distance a feature can return: a
+// lane tests a feature only when its ray enters that box nearer than its
 // current best, so a skipped feature could only have been rejected and
 // results are unchanged.  That holds for the features whose computed distance
 // is a slab entry of their own box or follows from it: plain boxes and prisms
@@ -48,8 +57,8 @@ static __device__ __noinline__ Feat featureAtOOL(LotDesc L, int g, int i) { retu
 // +-h.y and its caps lie at +-h.y, so its distance is inside the y slab; an
 // arch or ring keeps hits within +-h.z of its own frame (lot x or z by its
 // turn); an ellipsoid's root is not checked at all, so its box is unbounded.
-// (Testing quadrics alone in a culled run, or staging them apart, measured
-// slower: lanes then diverge inside the run.)
+// Cache entries also hold the union of these boxes over every run of kRun
+// records (the block-pooled trace culls by them).
 #ifndef STRATUM_COOP_RUN
 #define STRATUM_COOP_RUN 4
 #endif
@@ -106,10 +115,8 @@ struct CoopRay {
   unsigned long long stack;
   int node, qsteps, pend, state;
   int fresh;  // node's entry was just found nearer than best (by its parent's test)
-#if STRATUM_SPEC_LEAVES > 1
   unsigned queue;  // queued leaves of the current lot: group indices, 8 bits each, the head lowest
   int qn;
-#endif
 };
 
 SD int popNode(unsigned long long& stack) {
@@ -125,9 +132,7 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.state = active ? kEnterLot : kDone;
   r.stack = 0ull; r.node = 0; r.qsteps = 0; r.pend = 0; r.slot = 0; r.lcx = r.lcz = 0; r.fresh = 0;
   r.ddaSteps = 0;
-#if STRATUM_SPEC_LEAVES > 1
   r.queue = 0u; r.qn = 0;
-#endif
   if (!active) return;
   if (rd.y < -0.000001f) {
     float ground = -ro.y / rd.y;
@@ -178,9 +183,7 @@ SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __res
       continue;
     }
     if (r.node <= 0 || r.qsteps >= kNodes) {
-#if STRATUM_SPEC_LEAVES > 1
       if (r.qn > 0) { r.state = kLeafPending; r.pend = int(r.queue & 255u); break; }  // this lot's leaves first
-#endif
       r.state = kEnterLot;
       continue;
     }
@@ -204,7 +207,6 @@ SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __res
       else if (rh) r.node = right;
       else r.node = popNode(r.stack);
     } else {
-#if STRATUM_SPEC_LEAVES > 1
       if (near && r.node >= kGroups) {
         r.queue |= unsigned(r.node - kGroups) << (8 * r.qn);
         r.qn++;
@@ -212,9 +214,6 @@ SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __res
         if (r.qn == kSpec) { r.state = kLeafPending; r.pend = int(r.queue & 255u); break; }
         continue;
       }
-#else
-      if (near && r.node >= kGroups) { r.state = kLeafPending; r.pend = r.node - kGroups; break; }
-#endif
       r.node = popNode(r.stack);
     }
   }
@@ -247,20 +246,52 @@ SD Feat winnerFeature(const GroupCache& c, const float* __restrict__ W, int slot
   return featureAtOOL(L, g, i);
 }
 
-// Groups a warp stages and tests at once: lanes waiting on different groups
-// then test concurrently, each its own group's records.  One group at a time
-// measured fastest on the six benchmark poses (2, 3, 4 groups: frame 6 %, 16 %,
-// 27 % slower, the aerial view included), so the default is 1.
-#ifndef STRATUM_COOP_KEYS
-#define STRATUM_COOP_KEYS 1
-#endif
-constexpr int kKeys = STRATUM_COOP_KEYS;
 constexpr int kRunsPerGroup = (kEntryRecords + kRun - 1) / kRun;
-// Shared memory of one warp: kKeys groups of up to 56 records and their chunk boxes.
-struct WarpStage {
-  StagedFeat feats[kKeys][kEntryRecords];
-  ChunkBox boxes[kKeys][kRunsPerGroup];
-};
+// Shared memory of one warp: the records of the group it serves.
+struct WarpStage { StagedFeat feats[kEntryRecords]; };
+
+SD float warpMin(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+SD float warpMax(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// The rays a warp serves together, as one packet: they leave one point (the
+// camera in the lot's frame) with inverse directions between lo and hi, and
+// none wants a hit beyond `best`.
+struct Packet { f3 ro, lo, hi; float best; };
+
+// Whether some ray of the packet may hit this record nearer than its own best.
+// A ray's slab times of an axis are linear in its inverse direction, so over the
+// packet they lie between the extremes of the four products of the box's two
+// planes with the interval's two ends; a record is out when the latest of the
+// axes' earliest entries is past the earliest of their latest exits, or past
+// every ray's best.  The latter holds for boxes (masonry relief included, inside the
+// pad) and prisms only: quadrics and foliage are bounded by the box test alone.
+// The 0.025 m pad covers every rounding of this test and of the exact one: at
+// |ro| <= 2,100 m (a visited lot is at most 2,000 m along a ray) they sum to
+// less than 0.001 m.
+SD bool packetMayHit(const StagedFeat& s, const Packet& k) {
+  const int shape = (s.packed & 255) - 1;
+  const bool odd = (s.packed >> 16) & 1, base = shape == 3 || shape == 4;  // these stand on p.y
+  const float hx = (odd ? s.hz : s.hx) + 0.025f, hz = (odd ? s.hx : s.hz) + 0.025f, hy = s.hy + 0.025f;
+  const float ax = s.px - hx - k.ro.x, bx = s.px + hx - k.ro.x;
+  const float ay = (base ? s.py - 0.025f : s.py - hy) - k.ro.y, by = s.py + hy - k.ro.y;
+  const float az = s.pz - hz - k.ro.z, bz = s.pz + hz - k.ro.z;
+  const float x0 = ax * k.lo.x, x1 = ax * k.hi.x, x2 = bx * k.lo.x, x3 = bx * k.hi.x;
+  const float y0 = ay * k.lo.y, y1 = ay * k.hi.y, y2 = by * k.lo.y, y3 = by * k.hi.y;
+  const float z0 = az * k.lo.z, z1 = az * k.hi.z, z2 = bz * k.lo.z, z3 = bz * k.hi.z;
+  const float in = fmaxf(fmaxf(fminf(fminf(x0, x1), fminf(x2, x3)), fminf(fminf(y0, y1), fminf(y2, y3))),
+                         fminf(fminf(z0, z1), fminf(z2, z3)));
+  const float out = fminf(fminf(fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)), fmaxf(fmaxf(y0, y1), fmaxf(y2, y3))),
+                          fmaxf(fmaxf(z0, z1), fmaxf(z2, z3)));
+  return in <= out && out >= 0.001f && (in <= k.best || !(shape == 0 || shape == 3));
+}
 
 // Group records shared by the warps of one block, for a trace with no
 // table-wide group cache (the drop-in entry point).  Write-once for the
@@ -276,7 +307,6 @@ constexpr int kBlockEntries = STRATUM_BLOCK_CACHE_ENTRIES;
 static_assert(kBlockEntries >= 1 && kBlockEntries <= 32, "one lane per block-cache entry");
 struct BlockCache {
   StagedFeat feats[kBlockEntries][kEntryRecords];
-  ChunkBox boxes[kBlockEntries][kRunsPerGroup];
   int key[kBlockEntries];
   int count[kBlockEntries];
   volatile int ready[kBlockEntries];
@@ -298,25 +328,24 @@ SD int blockCacheFind(const BlockCache& bc, int key) {
   const unsigned m = __ballot_sync(0xffffffffu, hit);
   return m ? __ffs(m) - 1 : -1;
 }
-// Copy the group just staged in slot 0 of `ws` into a free entry, if any.  Warp-collective.
+// Copy the group just staged in `ws` into a free entry, if any.  Warp-collective.
 SD void blockCachePut(BlockCache& bc, const WarpStage& ws, int key, int count) {
   const int lane = int(threadIdx.x & 31);
   unsigned e = 0u;
   if (lane == 0) e = atomicAdd(&bc.next, 1u);
   e = __shfl_sync(0xffffffffu, e, 0);
   if (e >= unsigned(kBlockEntries)) return;
-  for (int k = lane; k < count; k += 32) bc.feats[e][k] = ws.feats[0][k];
-  if (lane < (count + kRun - 1) / kRun) bc.boxes[e][lane] = ws.boxes[0][lane];
+  for (int k = lane; k < count; k += 32) bc.feats[e][k] = ws.feats[k];
   if (lane == 0) { bc.key[e] = key; bc.count[e] = count; }
   __syncwarp();
   __threadfence_block();
   if (lane == 0) bc.ready[e] = 1;
 }
 
-// Stage one group into slot q of the warp's stage: its records from the group
-// cache, or built by the grammar (and stored when the cache gives an entry),
-// and the chunk boxes.  Warp-collective; returns the group's record count.
-SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key, WarpStage& ws, int q) {
+// Stage one group: its records from the group cache, or built by the grammar
+// (and stored when the cache gives an entry), and, where `boxes` is given, the
+// chunk boxes.  Warp-collective; returns the group's record count.
+SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key, StagedFeat* feats, ChunkBox* boxes) {
   const int lane = int(threadIdx.x & 31);
   const int slot = key >> 6, g = key & 63;
   // the directory word, the lot row, the entry's tag and its records in as few
@@ -333,16 +362,16 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
     StagedFeat r0{}, r1{};
     if (lane < count) r0 = cacheRecord(cache, e, lane);
     if (lane + 32 < count) r1 = cacheRecord(cache, e, lane + 32);
-    const int runs = (count + kRun - 1) / kRun;
+    const int runs = boxes ? (count + kRun - 1) / kRun : 0;
     float2 ba{}, bb{}, bc{};
     if (lane < runs) {
       const float2* bp = reinterpret_cast<const float2*>(entryBoxes(cache, uint32_t(e)) + lane * 6);
       ba = __ldg(bp); bb = __ldg(bp + 1); bc = __ldg(bp + 2);
     }
     if (__all_sync(0xffffffffu, same)) {  // records and chunk boxes as stored
-      if (lane < count) ws.feats[q][lane] = r0;
-      if (lane + 32 < count) ws.feats[q][lane + 32] = r1;
-      if (lane < runs) ws.boxes[q][lane] = ChunkBox{{ba.x, ba.y, bb.x}, {bb.y, bc.x, bc.y}};
+      if (lane < count) feats[lane] = r0;
+      if (lane + 32 < count) feats[lane + 32] = r1;
+      if (lane < runs) boxes[lane] = ChunkBox{{ba.x, ba.y, bb.x}, {bb.y, bc.x, bc.y}};
     } else {
       e = -1;
     }
@@ -358,9 +387,10 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
         StagedFeat s;
         stage(s, featureAtOOL(L, g, j));
         if (e >= 0) entryRecords(cache, uint32_t(e))[j] = s;
-        ws.feats[q][j] = s;
+        feats[j] = s;
         hitBox(unstage(s), lo, hi);
       }
+      if (e < 0 && !boxes) continue;
 #pragma unroll
       for (int o = 1; o < kRun; o <<= 1) {
         lo = vmin(lo, mk(__shfl_xor_sync(0xffffffffu, lo.x, o), __shfl_xor_sync(0xffffffffu, lo.y, o),
@@ -369,11 +399,10 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
                          __shfl_xor_sync(0xffffffffu, hi.z, o)));
       }
       if ((lane & (kRun - 1)) == 0 && j < count) {
-        const ChunkBox b = ChunkBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
-        ws.boxes[q][j / kRun] = b;
+        if (boxes) boxes[j / kRun] = ChunkBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
         if (e >= 0) {
           float* bp = entryBoxes(cache, uint32_t(e)) + (j / kRun) * 6;
-          bp[0] = b.lo[0]; bp[1] = b.lo[1]; bp[2] = b.lo[2]; bp[3] = b.hi[0]; bp[4] = b.hi[1]; bp[5] = b.hi[2];
+          bp[0] = lo.x; bp[1] = lo.y; bp[2] = lo.z; bp[3] = hi.x; bp[4] = hi.y; bp[5] = hi.z;
         }
       }
     }
@@ -399,76 +428,69 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
     coopAdvance(r, W, N, o0, o2);
     unsigned pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
     if (!pending) break;  // every lane is done (lanes only stop advancing at a leaf or when done)
-#if STRATUM_SPEC_LEAVES > 1
-    static_assert(kKeys == 1, "queued leaves are served one group at a time");
 #pragma unroll 1
     while (pending) {
+      // the first pending lane's (lot, group), for every lane that waits on it
       const int myKey = (r.slot << 6) | r.pend;
-#else
-    const int myKey = (r.slot << 6) | r.pend;
-#pragma unroll 1
-    while (pending) {
-#endif
-      // up to kKeys distinct keys of the pending lanes (first pending lane's
-      // key first), staged one after another
-      unsigned batch = 0u;
-      int myq = -1, myCount = 0;
-      const StagedFeat* myFeats = nullptr;
-      const ChunkBox* myBoxes = nullptr;
-#pragma unroll
-      for (int q = 0; q < kKeys; q++) {
-        const unsigned rem = pending & ~batch;
-        if (!rem) break;
-        const int key = __shfl_sync(0xffffffffu, myKey, __ffs(rem) - 1);
-        const unsigned peers = __ballot_sync(0xffffffffu, r.state == kLeafPending && myKey == key);
-        batch |= peers;
-        if constexpr (kBlockCache) {
-          int count;
-          const StagedFeat* feats = ws.feats[q];
-          const ChunkBox* boxes = ws.boxes[q];
-          const int e = blockCacheFind(*bc, key);
-          if (e >= 0) {  // built earlier by a warp of this block
-            count = bc->count[e];
-            feats = bc->feats[e];
-            boxes = bc->boxes[e];
-          } else {
-            count = stageGroup(W, cache, key, ws, q);
-            if (q == 0) {
-              __syncwarp();
-              blockCachePut(*bc, ws, key, count);
-            }
-          }
-          if ((peers >> lane) & 1u) { myq = q; myCount = count; myFeats = feats; myBoxes = boxes; }
+      const int key = __shfl_sync(0xffffffffu, myKey, __ffs(pending) - 1);
+      const bool peer = r.state == kLeafPending && myKey == key;
+      const unsigned peers = __ballot_sync(0xffffffffu, peer);
+      int count;
+      const StagedFeat* feats = ws.feats;
+      if constexpr (kBlockCache) {
+        const int e = blockCacheFind(*bc, key);
+        if (e >= 0) {  // built earlier by a warp of this block
+          count = bc->count[e];
+          feats = bc->feats[e];
+          __syncwarp();
         } else {
-          const int count = stageGroup(W, cache, key, ws, q);
-          if ((peers >> lane) & 1u) { myq = q; myCount = count; }
+          count = stageGroup(W, cache, key, ws.feats, nullptr);
+          __syncwarp();
+          blockCachePut(*bc, ws, key, count);
         }
+      } else {
+        count = stageGroup(W, cache, key, ws.feats, nullptr);
+        __syncwarp();
       }
-      __syncwarp();
-      // every waiting lane tests its own group's records in index order
-      if (myq >= 0) {
+      // lanes are records: which of them can any peer's ray hit
+      const float big = 1e30f;
+      Packet pk;
+      const int src = __ffs(peers) - 1;
+      pk.ro = mk(__shfl_sync(0xffffffffu, r.lr.x, src), __shfl_sync(0xffffffffu, r.lr.y, src),
+                 __shfl_sync(0xffffffffu, r.lr.z, src));
+      pk.lo = mk(warpMin(peer ? r.inv0.x : big), warpMin(peer ? r.inv0.y : big), warpMin(peer ? r.inv0.z : big));
+      pk.hi = mk(warpMax(peer ? r.inv0.x : -big), warpMax(peer ? r.inv0.y : -big), warpMax(peer ? r.inv0.z : -big));
+      pk.best = warpMax(peer ? r.best : 0.0f);
+      const unsigned m0 = __ballot_sync(0xffffffffu, lane < count && packetMayHit(feats[lane], pk));
+      const unsigned m1 =
+          count <= 32 ? 0u : __ballot_sync(0xffffffffu, lane + 32 < count && packetMayHit(feats[lane + 32], pk));
+      if (peer) {
+        // those records in index order: the first feature wins ties
         const int g = r.pend;
+        unsigned mlo = m0, mhi = m1;
 #pragma unroll 1
-        for (int c = 0; c * kRun < myCount; c++) {
-          const ChunkBox b = kBlockCache ? myBoxes[c] : ws.boxes[myq][c];
-          const Span cr = slabInv(r.lr, r.inv0, mk(b.lo[0], b.lo[1], b.lo[2]), mk(b.hi[0], b.hi[1], b.hi[2]));
-          if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // no feature of the run can win
-          const int kEnd = min(myCount, (c + 1) * kRun);
-#pragma unroll 1
-          for (int k = c * kRun; k < kEnd; k++) {
-            const Feat f = unstage(kBlockCache ? myFeats[k] : ws.feats[myq][k]);
-            const bool odd = f.turn % 2 == 1;
-            const f3 inv = odd ? inv1Of(r) : r.inv0, p = intoFeature(r.lr - f.p, f.turn);
-            const Span rg = featureSlab(f, p, inv);
-            if (featureSlabMiss(f, rg)) continue;
-            const f3 d = odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld;
-            const float th = featureAfterSlab(f, r.lr, r.ld, p, d, inv, rg, r.cone);
-            if (th > 0.001f && th < r.best) {  // index order: the first feature wins ties
-              r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
-            }
+        while (mlo | mhi) {
+          const int k = mlo ? __ffs(mlo) - 1 : __ffs(mhi) + 31;
+          if (mlo) mlo &= mlo - 1u; else mhi &= mhi - 1u;
+          const Feat f = unstage(feats[k]);
+          const bool odd = f.turn % 2 == 1;
+          const f3 inv = odd ? inv1Of(r) : r.inv0, p = intoFeature(r.lr - f.p, f.turn);
+          const Span rg = featureSlab(f, p, inv);
+          if (featureSlabMiss(f, rg)) continue;
+          float th;
+          if (plainBox(f)) {
+            th = plainBoxHit(rg);
+          } else {
+            f3 lo, hi;
+            hitBox(f, lo, hi);
+            const Span cr = slabInv(r.lr, r.inv0, lo, hi);
+            if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
+            th = featureAfterSlabOOL(f, r.lr, r.ld, p, odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld, inv, r.cone);
+          }
+          if (th > 0.001f && th < r.best) {
+            r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
           }
         }
-#if STRATUM_SPEC_LEAVES > 1
         // the next queued leaf that can still win (its node tested against
         // the best just found, as the reference tests it when it gets there)
         r.queue >>= 8;
@@ -484,14 +506,6 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
       __syncwarp();
       pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
     }
-#else
-        r.state = kInLot;
-        r.node = popNode(r.stack);
-      }
-      __syncwarp();
-      pending &= ~batch;
-    }
-#endif
   }
   TraceResult out;
   out.t = r.best; out.fid = r.fid; out.material = 10; out.seed = 0.0f; out.slot = -1;

@@ -19,11 +19,14 @@
 
 namespace st {
 
-static_assert(kSpec > 1 && kKeys == 1, "the pooled trace serves queued leaves one group at a time");
-
+// Shared memory of one warp: the records of the group it serves and their chunk boxes.
+struct PoolStage {
+  StagedFeat feats[kEntryRecords];
+  ChunkBox boxes[kRunsPerGroup];
+};
 template <int P>
 struct PoolShared {
-  WarpStage stage[P];
+  PoolStage stage[P];
   float lr[3][P * 32], ld[3][P * 32], inv[3][P * 32];
   float best[P * 32], cone[P * 32];
   int key[P * 32];  // pending head (view << 20 | slot << 6 | group), or -1
@@ -37,7 +40,7 @@ SD int poolWarpOf(int key) { return int((unsigned(key) * 2654435761u) >> 16) % P
 // One ray of the block against the group staged in `ws` (the record loop of
 // traceWarp, on the ray's state in shared memory).
 template <int P>
-SD void poolTest(PoolShared<P>& sh, int j, const WarpStage& ws, int count, int g) {
+SD void poolTest(PoolShared<P>& sh, int j, const PoolStage& ws, int count, int g) {
   const f3 lr = mk(sh.lr[0][j], sh.lr[1][j], sh.lr[2][j]);
   const f3 ld = mk(sh.ld[0][j], sh.ld[1][j], sh.ld[2][j]);
   const f3 inv0 = mk(sh.inv[0][j], sh.inv[1][j], sh.inv[2][j]);
@@ -46,13 +49,13 @@ SD void poolTest(PoolShared<P>& sh, int j, const WarpStage& ws, int count, int g
   int fid = -1;
 #pragma unroll 1
   for (int c = 0; c * kRun < count; c++) {
-    const ChunkBox b = ws.boxes[0][c];
+    const ChunkBox b = ws.boxes[c];
     const Span cr = slabInv(lr, inv0, mk(b.lo[0], b.lo[1], b.lo[2]), mk(b.hi[0], b.hi[1], b.hi[2]));
     if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > best) continue;  // no feature of the run can win
     const int kEnd = min(count, (c + 1) * kRun);
 #pragma unroll 1
     for (int k = c * kRun; k < kEnd; k++) {
-      const Feat f = unstage(ws.feats[0][k]);
+      const Feat f = unstage(ws.feats[k]);
       const bool odd = f.turn % 2 == 1;
       const f3 inv = odd ? mk(inv0.z, inv0.y, ld.x == 0.0f ? guardedInv(-ld.x) : -inv0.x) : inv0;
       const f3 p = intoFeature(lr - f.p, f.turn);
@@ -100,8 +103,8 @@ SD void poolServe(PoolShared<P>& sh, const stratum_view* __restrict__ V) {
       total += __popc(wait[p]);
     }
     const int v = key >> 20, slot = (key >> 6) & (kLots - 1), g = key & 63;
-    WarpStage& ws = sh.stage[warp];
-    const int count = stageGroup(V[v].World, groupCache(V[v].Groups), (slot << 6) | g, ws, 0);
+    PoolStage& ws = sh.stage[warp];
+    const int count = stageGroup(V[v].World, groupCache(V[v].Groups), (slot << 6) | g, ws.feats, ws.boxes);
     __syncwarp();
     // the waiting rays, compacted: lane i takes the i-th of each 32
 #pragma unroll 1
