@@ -61,6 +61,11 @@ static __device__ __noinline__ float foliageHit(f3 ro, f3 rd, f3 centre, f3 radi
 // (geometry.cu:82-89).  Called only for tall stone/brick boxes.
 static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f3 d, float t, float cone) {
   const f3 h = f.h;
+  // Beyond freqWeight's cut-off (t * cone >= 0.0275: 23 m at 900 rows) the relief
+  // is multiplied by exactly 0 and every step leaves t where it is; without this
+  // return the four height-field steps of far walls took 13 % of the six-view
+  // 1600x900 trace (6.80 -> 5.91 ms, aerial pose 2.89 -> 2.39 ms).
+  if (freqWeight(t * cone, 40.0f) == 0.0f) return t;
   f3 hp = p + d * t;
   float ex = fabsf(fabsf(hp.x) - h.x), ez = fabsf(fabsf(hp.z) - h.z);
   if (fabsf(fabsf(hp.y) - h.y) > 0.01f) {
