@@ -103,8 +103,9 @@ int stratum_commitPages(const unsigned* Queue, unsigned* Args, stratum_stream_t 
 int stratum_buildBVH(const unsigned* Queue, const float* World, float* Nodes, stratum_stream_t stream);
 
 /* ---- whole frame (the ordered sequence of src/engine.js:67-83) ------------ */
-/* stepCamera, clearQueue, prepareLots, planBounds, buildBVH, then trace and
- * shade in 64-row strips and resolveFrame.  `Args` may be NULL. */
+/* stepCamera, clearQueue, prepareLots, planBounds, buildBVH, then
+ * tracePrimary, shadePixels (all rows in one launch each) and resolveFrame.
+ * `Args` may be NULL. */
 int stratum_frame(float* C, unsigned* Origin, const float* I, float dt, float* World, unsigned* Tags, float* Nodes,
                   unsigned* Queue, unsigned* Args, float* Hit, float* Surface, float* Linear, float* History,
                   unsigned* Pixels, int width, int height, int draw, stratum_stream_t stream);

@@ -17,7 +17,6 @@ from . import (BUILD_CHUNK, BUILD_CHUNKS, GROUP_NODES, LOT_FLOATS, WORLD_LOTS, c
 
 BUILD_ID = "infinite-shared-grammar-1"
 STAGES = ["World descriptors", "Bounds refresh", "Exact visibility", "Materials + light", "Resolve"]
-ROWS = 64
 
 
 class Engine:
@@ -109,12 +108,10 @@ class Engine:
 
     def draw(self):
         b, s, w, h = self.buffers, self._s(), self.width, self.height
-        for y in range(0, h, ROWS):
-            call("stratum_tracePrimary", ptr(b["World"]), ptr(b["Nodes"]), ptr(b["Origin"]), ptr(b["C"]),
-                 ptr(b["Hit"]), ptr(b["Surface"]), w, h, y, min(ROWS, h - y), s)
-        for y in range(0, h, ROWS):
-            call("stratum_shadePixels", ptr(b["World"]), ptr(b["Origin"]), ptr(b["C"]), ptr(b["Hit"]),
-                 ptr(b["Surface"]), ptr(b["Linear"]), w, h, y, min(ROWS, h - y), s)
+        call("stratum_tracePrimary", ptr(b["World"]), ptr(b["Nodes"]), ptr(b["Origin"]), ptr(b["C"]),
+             ptr(b["Hit"]), ptr(b["Surface"]), w, h, 0, h, s)
+        call("stratum_shadePixels", ptr(b["World"]), ptr(b["Origin"]), ptr(b["C"]), ptr(b["Hit"]),
+             ptr(b["Surface"]), ptr(b["Linear"]), w, h, 0, h, s)
         call("stratum_resolveFrame", ptr(b["Linear"]), ptr(b["History"]), ptr(b["Pixels"]), ptr(b["C"]),
              ptr(b["Hit"]), ptr(b["Surface"]), w, h, s)
 
