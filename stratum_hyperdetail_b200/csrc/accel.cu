@@ -17,11 +17,11 @@ __global__ void __launch_bounds__(64) buildGroupBoundsK(const uint32_t* Q, const
   int slot = int(Q[q + 1]);
   if (slot < 0 || slot >= kLots) return;
   LotDesc lot = loadLot(W, slot);
-  float n[8];
-  leafBounds(lot, g, n);
+  float n[7];
+  groupBounds(lot, regularLot(lot), g, n);
   float4* dst = reinterpret_cast<float4*>(N + (size_t(slot) * kNodes + kGroups + g) * 8);
   dst[0] = make_float4(n[0], n[1], n[2], n[3]);
-  dst[1] = make_float4(n[4], n[5], n[6], n[7]);
+  dst[1] = make_float4(n[4], n[5], n[6], float(g));
 }
 
 __global__ void reduceGroupBoundsK(const uint32_t* Q, float* N, int first, int queueBase) {
@@ -37,9 +37,9 @@ __global__ void reduceGroupBoundsK(const uint32_t* Q, float* N, int first, int q
   b[7] = 0.0f;
 }
 
-__global__ void __launch_bounds__(64) buildLotHierarchyK(const uint32_t* Q, const float* W, float* N) {
-  __shared__ __align__(16) float sm[kNodes][8];
-  buildQueue(Q, W, N, int(blockIdx.x), int(gridDim.x), sm);
+__global__ void __launch_bounds__(kBuildThreads, kBuildBlocks) buildLotHierarchyK(const uint32_t* Q, const float* W, float* N) {
+  __shared__ BuildShared sh;
+  buildQueue(Q, W, N, int(blockIdx.x), int(gridDim.x), sh);
 }
 
 }  // namespace st
@@ -58,8 +58,8 @@ int stratumHierarchyGrid() {
   std::call_once(once[dev], [dev] {
     int sms = 148, per = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, buildLotHierarchyK, 64, 0);
-    blocks[dev] = sms * (per > 0 ? per : 8);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, buildLotHierarchyK, kBuildThreads, 0);
+    blocks[dev] = sms * (per > 0 ? per : 2);
   });
   return blocks[dev];
 }
@@ -80,7 +80,7 @@ int stratum_reduceGroupBounds(const unsigned* Queue, float* Nodes, int first, in
 }
 int stratum_buildBVH(const unsigned* Queue, const float* World, float* Nodes, stratum_stream_t stream) {
   if (!Queue || !World || !Nodes) return STRATUM_EINVAL;
-  buildLotHierarchyK<<<stratumHierarchyGrid(), 64, 0, asStream(stream)>>>(Queue, World, Nodes);
+  buildLotHierarchyK<<<stratumHierarchyGrid(), kBuildThreads, 0, asStream(stream)>>>(Queue, World, Nodes);
   return launchStatus();
 }
 

@@ -73,11 +73,11 @@ __global__ void refreshViewsK(const stratum_view* __restrict__ V, int n) {
   refreshSlot(slot, w.Origin, int(w.C[14]), w.World, w.Tags, w.Queue);
 }
 
-__global__ void __launch_bounds__(64) buildViewsK(const stratum_view* __restrict__ V, int n) {
-  __shared__ __align__(16) float sm[kNodes][8];
+__global__ void __launch_bounds__(kBuildThreads, kBuildBlocks) buildViewsK(const stratum_view* __restrict__ V, int n) {
+  __shared__ BuildShared sh;
   const int v = int(blockIdx.y);
   if (v >= n) return;
-  buildQueue(V[v].Queue, V[v].World, V[v].Nodes, int(blockIdx.x), int(gridDim.x), sm);
+  buildQueue(V[v].Queue, V[v].World, V[v].Nodes, int(blockIdx.x), int(gridDim.x), sh);
 }
 
 // The directory of a group cache whose reset the prologue just decided.
@@ -522,7 +522,7 @@ int stratum_refreshViews(stratum_view* views, int n, stratum_stream_t stream) {
 int stratum_buildViews(stratum_view* views, int n, stratum_stream_t stream) {
   if (!views || n <= 0 || n > 65535) return STRATUM_EINVAL;
   int per = stratumHierarchyGrid() / n;
-  buildViewsK<<<dim3(per < 16 ? 16 : per, n), 64, 0, asStream(stream)>>>(views, n);
+  buildViewsK<<<dim3(per < 16 ? 16 : per, n), kBuildThreads, 0, asStream(stream)>>>(views, n);
   return launchStatus();
 }
 int stratum_traceViews(stratum_view* views, int n, void* scratch, unsigned long long scratchBytes,

@@ -255,4 +255,16 @@ HD f3 toLot(f3 p, int turn) {
 }
 HD f3 fromLot(f3 p, int turn) { return toLot(p, (4 - turn) % 4); }
 
+// Least and greatest value over a full warp (every lane calls).
+SD float warpMin(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+SD float warpMax(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 }  // namespace st

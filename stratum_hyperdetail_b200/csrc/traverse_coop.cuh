@@ -250,17 +250,6 @@ constexpr int kRunsPerGroup = (kEntryRecords + kRun - 1) / kRun;
 // Shared memory of one warp: the records of the group it serves.
 struct WarpStage { StagedFeat feats[kEntryRecords]; };
 
-SD float warpMin(float v) {
-  float r;
-  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-SD float warpMax(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-
 // The rays a warp serves together, as one packet: they leave one point (the
 // camera in the lot's frame) with inverse directions between lo and hi, and
 // none wants a hit beyond `best`.
