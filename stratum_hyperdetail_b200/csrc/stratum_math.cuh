@@ -162,8 +162,18 @@ HD float masonryHeight(float u, float v, int material) {
   float x = fract(u / bw + float(imod(row, 2)) * 0.5f), y = fract(v / bh);
   float edge = fminf(fminf(x, 1.0f - x) * bw, fminf(y, 1.0f - y) * bh);
   float grain = noise2(u * 24.0f, v * 24.0f);
-  float chipped = edge - 0.006f * smooth(0.34f, 0.73f, noise2(u * 117.0f, v * 117.0f));
-  return -0.018f * (1.0f - smooth(0.008f, 0.023f, chipped)) + 0.0025f * grain;
+  // The chipping noise takes up to 0.006 m off the edge distance before the step
+  // from 0.008 to 0.023 m: outside 0.008..0.029 m the step is exactly 0 or 1
+  // whatever the noise (74 % of a brick, 86 % of a stone).
+  float mortar = 1.0f;
+  if (edge > 0.008f) {
+    mortar = 0.0f;
+    if (!(edge - 0.006f >= 0.023f)) {
+      float chipped = edge - 0.006f * smooth(0.34f, 0.73f, noise2(u * 117.0f, v * 117.0f));
+      mortar = 1.0f - smooth(0.008f, 0.023f, chipped);
+    }
+  }
+  return -0.018f * mortar + 0.0025f * grain;
 }
 HD uint32_t packRGBA8(f3 c) {
   uint32_t r = uint32_t(sat(c.x) * 255.0f), g = uint32_t(sat(c.y) * 255.0f), b = uint32_t(sat(c.z) * 255.0f);

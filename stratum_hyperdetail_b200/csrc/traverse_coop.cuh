@@ -470,11 +470,16 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
           if (plainBox(f)) {
             th = plainBoxHit(rg);
           } else {
-            f3 lo, hi;
-            hitBox(f, lo, hi);
-            const Span cr = slabInv(r.lr, r.inv0, lo, hi);
-            if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
-            th = featureAfterSlabOOL(f, r.lr, r.ld, p, odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld, inv, r.cone);
+            const f3 d = odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld;
+            if (f.shape == 3) {  // its distance is never before the slab's entry
+              if (rg.lo > r.best || prismMiss(f, p, d, rg)) continue;
+            } else {
+              f3 lo, hi;
+              hitBox(f, lo, hi);
+              const Span cr = slabInv(r.lr, r.inv0, lo, hi);
+              if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
+            }
+            th = featureInSlabOOL(f, r.lr, r.ld, p, d, rg, r.cone);
           }
           if (th > 0.001f && th < r.best) {
             r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;

@@ -62,7 +62,7 @@ SD void poolTest(PoolShared<P>& sh, int j, const PoolStage& ws, int count, int g
       const Span rg = featureSlab(f, p, inv);
       if (featureSlabMiss(f, rg)) continue;
       const f3 d = odd ? mk(ld.z, ld.y, -ld.x) : ld;
-      const float th = featureAfterSlab(f, lr, ld, p, d, inv, rg, cone);
+      const float th = featureAfterSlab(f, lr, ld, p, d, rg, cone);
       if (th > 0.001f && th < best) {  // index order: the first feature wins ties
         best = th;
         fid = g * kMaxFeatures + k;
