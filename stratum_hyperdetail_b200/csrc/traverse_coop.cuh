@@ -3,32 +3,39 @@
 // Same algorithm as traverse.cuh (kernels/trace.cu of the reference), same
 // results bit for bit, organised for a warp of 32 coherent rays (one 8x4 tile):
 //
-//  * each lane advances its own ray -- lot DDA, then the near-first descent of
-//    the lot's hierarchy -- until it reaches a leaf (a group) that must be
-//    evaluated, or finishes;
-//  * the warp then evaluates pending leaves one distinct (lot, group) key at a
-//    time: the group's records are staged in shared memory, one per lane --
-//    loaded from the table's group cache (group_cache.cuh) when it holds the
-//    group, else built by the random-access grammar (grammar_ra.cuh) and, when
-//    the cache has room, stored there for every later evaluation.  The lanes
-//    then stand for records: each tests its one or two records against all the
-//    waiting rays at once, taken as a packet (packetMayHit).  Most evaluations
-//    end here (63 % of them on the street pose, 38 % on the aerial one, keep no
-//    record; the others keep 2-5 of up to 56), and every lane waiting on the key
-//    tests the records kept, in index order, with one inlined intersection
-//    routine and its precomputed inverse directions.  What bounds the kernel is
-//    instruction issue and latency: walking the waiting rays through all the
-//    records behind one box test per run of four took 1,000 (aerial) to 2,500
-//    (street) instructions per evaluation, this takes about 250; six-view
-//    1600x900 trace 7.61 -> 6.80 ms (street 1.76 -> 1.36, aerial 3.15 -> 2.89).
-//    One lane per (ray, record) pair by ballots over every waiting ray (its own
-//    candidate mask per lane) measured 7.27 ms;
+//  * each lane steps its own lot DDA to the next lot whose root it enters;
+//  * the warp takes the lots its lanes wait in one at a time.  Lanes stand for
+//    leaves: all 64 groups of the lot are tested at once against the waiting rays,
+//    taken as a packet (packetMayEnter), and each ray then tests the few leaves
+//    left (3-6) itself and orders its own by the reference's near-first descent,
+//    which needs the hierarchy only where the paths to two of its leaves part;
+//  * when every lane waits on a leaf or is done, the warp evaluates one distinct
+//    (lot, group) at a time for all the lanes that wait on it.  Its records come
+//    from the table's group cache (group_cache.cuh), the block's table (the
+//    drop-in), or the random-access grammar (grammar_ra.cuh), which stores them
+//    when the cache has room.  Lanes now stand for records and test them against
+//    the packet (packetMayHit): most evaluations end there (63 % on the street pose,
+//    38 % on the aerial one, keep no record, the others 2-5 of up to 56), and the
+//    waiting lanes test the records kept, in index order, with one inlined
+//    intersection routine;
 //  * the winner's normal, material and seed are recomputed once per ray.
+//
+// What bounds the kernel is instruction issue and latency, and code size beyond
+// the instruction cache (108 KB here; at 150 KB the aerial pose took twice as long
+// on instruction fetch).  Six-view 1600x900 trace: each ray walking all records of
+// a group behind a box test per run of four, 1,000 (aerial) to 2,500 (street)
+// instructions an evaluation, 7.61 ms; records by packet 6.80 ms; without the
+// arithmetic of masonry relief and prisms that is certain to come to nothing
+// 5.72 ms; leaves by packet instead of a 25-node descent per lane 4.76 ms (street
+// 1.18 -> 0.82, aerial 2.29 -> 2.11).  Measured and left out: per-ray candidate
+// masks by a ballot per (ray, record) 7.27 ms against 6.80; culling a lot's
+// records for all its leaves before the rays order them (street 0.86, aerial 4.43:
+// it evaluates groups no ray reaches, which no longer fit the cache); 640 and 768
+// threads per SM (spills) 5.16 and 5.01 ms against 4.86.
 //
 // Each lane's leaves are visited in the reference's order and each test sees
 // the same running best, so identity, distance and normal equal the
-// per-thread traversal exactly.  The per-lot hierarchy stack is packed into
-// one 64-bit word (7 bits per node, at most 6 entries).
+// per-thread traversal exactly.
 #pragma once
 #include "geometry.cuh"
 #include "grammar_ra.cuh"
@@ -86,19 +93,49 @@ SD void hitBox(const Feat& f, f3& lo, f3& hi) {
   }
 }
 
-enum LaneState : int { kEnterLot = 0, kInLot = 1, kLeafPending = 2, kDone = 3 };
+// The rays a warp serves together, as one packet: they leave one point (the
+// camera in the lot's frame) with inverse directions between lo and hi, and
+// none wants a hit beyond `best`.
+struct Packet { f3 ro, lo, hi; float best; };
 
-// Leaves a lane may find ahead in its lot before the warp evaluates them.  With
-// more than one, a lane that reaches a leaf keeps walking the lot's hierarchy
-// (near-first, against the best it has) and queues up to this many leaves; each
-// queued leaf is tested again against the lane's best when it comes up, so the
-// lane evaluates exactly the reference's leaves in the reference's order (a
-// leaf that passes has ancestors that pass: parents bound their children).
-#ifndef STRATUM_SPEC_LEAVES
-#define STRATUM_SPEC_LEAVES 4
-#endif
-constexpr int kSpec = STRATUM_SPEC_LEAVES;
-static_assert(kSpec >= 1 && kSpec <= 4, "up to four queued leaves (8 bits each in one word)");
+// Whether some ray of the packet may hit this record nearer than its own best.
+// A ray's slab times of an axis are linear in its inverse direction, so over the
+// packet they lie between the extremes of the four products of the box's two
+// planes with the interval's two ends; a record is out when the latest of the
+// axes' earliest entries is past the earliest of their latest exits, or past
+// every ray's best.  The latter holds for boxes (masonry relief included, inside the
+// pad) and prisms only: quadrics and foliage are bounded by the box test alone.
+// The 0.025 m pad covers every rounding of this test and of the exact one: at
+// |ro| <= 2,100 m (a visited lot is at most 2,000 m along a ray) they sum to
+// less than 0.001 m.
+SD bool packetEnters(const Packet& k, f3 lo, f3 hi, float& in) {
+  const float ax = lo.x - k.ro.x, bx = hi.x - k.ro.x, ay = lo.y - k.ro.y, by = hi.y - k.ro.y;
+  const float az = lo.z - k.ro.z, bz = hi.z - k.ro.z;
+  const float x0 = ax * k.lo.x, x1 = ax * k.hi.x, x2 = bx * k.lo.x, x3 = bx * k.hi.x;
+  const float y0 = ay * k.lo.y, y1 = ay * k.hi.y, y2 = by * k.lo.y, y3 = by * k.hi.y;
+  const float z0 = az * k.lo.z, z1 = az * k.hi.z, z2 = bz * k.lo.z, z3 = bz * k.hi.z;
+  in = fmaxf(fmaxf(fminf(fminf(x0, x1), fminf(x2, x3)), fminf(fminf(y0, y1), fminf(y2, y3))),
+             fminf(fminf(z0, z1), fminf(z2, z3)));
+  const float out = fminf(fminf(fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)), fmaxf(fmaxf(y0, y1), fmaxf(y2, y3))),
+                          fmaxf(fmaxf(z0, z1), fmaxf(z2, z3)));
+  return in <= out && out >= 0.001f;
+}
+// Whether some ray may enter this node's box nearer than its own best.
+SD bool packetMayEnter(float4 a, float4 b, const Packet& k) {
+  const float pad = 0.01f;
+  float in;
+  return packetEnters(k, mk(a.x - pad, a.y - pad, a.z - pad), mk(b.x + pad, b.y + pad, b.z + pad), in) && in <= k.best;
+}
+SD bool packetMayHit(const StagedFeat& s, const Packet& k) {
+  const int shape = (s.packed & 255) - 1;
+  const bool odd = (s.packed >> 16) & 1, base = shape == 3 || shape == 4;  // these stand on p.y
+  const float hx = (odd ? s.hz : s.hx) + 0.025f, hz = (odd ? s.hx : s.hz) + 0.025f, hy = s.hy + 0.025f;
+  float in;
+  return packetEnters(k, mk(s.px - hx, base ? s.py - 0.025f : s.py - hy, s.pz - hz), mk(s.px + hx, s.py + hy, s.pz + hz), in) &&
+         (in <= k.best || !(shape == 0 || shape == 3));
+}
+
+enum LaneState : int { kEnterLot = 0, kLotPending = 1, kLeafPending = 2, kDone = 3 };
 
 struct CoopRay {
   // ray and result
@@ -111,28 +148,21 @@ struct CoopRay {
   // current lot
   int slot, lcx, lcz;
   f3 lr, ld, inv0;
-  // hierarchy walk
-  unsigned long long stack;
-  int node, qsteps, pend, state;
-  int fresh;  // node's entry was just found nearer than best (by its parent's test)
-  unsigned queue;  // queued leaves of the current lot: group indices, 8 bits each, the head lowest
-  int qn;
+  // leaves (groups) of the current lot still to be evaluated, the inner nodes whose
+  // right child comes first, the leaf that is next, and whether best has changed
+  // since the leaves were found
+  unsigned long long leaves, rightFirst;
+  int pend, state;
+  bool moved;
 };
-
-SD int popNode(unsigned long long& stack) {
-  int n = int(stack & 127ull);
-  stack >>= 7;
-  return n;
-}
 
 // Ray set-up: ground plane and vertical slab (trace.cu:33-45).
 SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.ro = ro; r.rd = rd; r.cone = cone;
   r.best = kFar; r.fid = kSkyId; r.wslot = -1; r.wcx = r.wcz = 0;
   r.state = active ? kEnterLot : kDone;
-  r.stack = 0ull; r.node = 0; r.qsteps = 0; r.pend = 0; r.slot = 0; r.lcx = r.lcz = 0; r.fresh = 0;
+  r.leaves = r.rightFirst = 0ull; r.moved = false; r.pend = 0; r.slot = 0; r.lcx = r.lcz = 0;
   r.ddaSteps = 0;
-  r.queue = 0u; r.qn = 0;
   if (!active) return;
   if (rd.y < -0.000001f) {
     float ground = -ro.y / rd.y;
@@ -159,64 +189,86 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.dz = kCell * fabsf(iz);
 }
 
-// Advance one lane until it needs a leaf evaluated or is done.
-SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __restrict__ N, uint32_t o0, uint32_t o2) {
+// Inner node where the paths to two leaves part.
+SD int forkOf(int a, int b) { return (kGroups + a) >> (32 - __clz(a ^ b)); }
+
+// The order of the lane's leaves: the reference's near-first descent decides
+// between two leaves at the node where their paths part, by the entries of its
+// two children (ties go right).  Those nodes are the forks of neighbouring
+// leaves; nothing else of the hierarchy is read.
+SD void orderLeaves(CoopRay& r, const float4* __restrict__ N) {
+  const int base = r.slot * kNodes;
+  r.rightFirst = 0ull;
+  r.moved = false;
+  unsigned long long rest = r.leaves;
 #pragma unroll 1
-  while (r.state == kEnterLot || r.state == kInLot) {
-    if (r.state == kEnterLot) {
-      if (r.ddaSteps >= 160 || r.t > r.best || r.t > r.farT || r.t > kFar) { r.state = kDone; break; }
-      r.ddaSteps++;
-      r.slot = tableSlot(o0, o2, r.cx, r.cz);
-      r.lcx = r.cx; r.lcz = r.cz;
-      const float4 c = __ldg(reinterpret_cast<const float4*>(W + r.slot * kLotFloats) + 2);  // roofScale, turn, ox, oz
-      const int turn = int(c.y);
-      f3 cp = mk(float(r.cx) * kCell + c.z, 0.0f, float(r.cz) * kCell + c.w);
-      r.lr = toLot(r.ro - cp, turn);
-      r.ld = toLot(r.rd, turn);
-      r.inv0 = invDir(r.ld);
-      // the DDA steps to the next cell now; the reference does it after the
-      // lot's query, and the next test reads only t and the (later) best
-      if (r.tx < r.tz) { r.t = r.tx; r.tx += r.dx; r.cx += r.sx; } else { r.t = r.tz; r.tz += r.dz; r.cz += r.sz; }
-      if (nodeEntry(N, r.slot * kNodes + 1, r.lr, r.inv0, r.best) < r.best) {
-        r.state = kInLot; r.node = 1; r.stack = 0ull; r.qsteps = 0; r.fresh = 1;
-      }
-      continue;
+  while (rest & (rest - 1ull)) {
+    const int a = __ffsll(rest) - 1;
+    rest &= rest - 1ull;
+    const int fork = forkOf(a, __ffsll(rest) - 1);
+    const float ln = nodeEntry(N, base + 2 * fork, r.lr, r.inv0, r.best);
+    const float rn = nodeEntry(N, base + 2 * fork + 1, r.lr, r.inv0, r.best);
+    if (!(ln < rn)) r.rightFirst |= 1ull << fork;
+  }
+}
+
+// Take the lane's next leaf in that order, or send it to its next lot.  Once best
+// has moved a leaf is tested again and dropped when it has fallen behind, as the
+// reference drops it when it gets there: best only falls and a node's entry is
+// never after its children's, so a leaf is visited exactly when its own test
+// passes then.
+SD void nextLeaf(CoopRay& r, const float4* __restrict__ N) {
+  r.state = kEnterLot;
+#pragma unroll 1
+  while (r.leaves) {
+    unsigned long long cur = r.leaves;
+#pragma unroll 1
+    while (cur & (cur - 1ull)) {
+      const int first = __ffsll(cur) - 1, last = 63 - __clzll(cur), level = 31 - __clz(first ^ last);
+      const unsigned long long below = cur & ((1ull << (((first >> level) | 1) << level)) - 1ull);
+      cur = (r.rightFirst >> ((kGroups + first) >> (level + 1))) & 1ull ? cur ^ below : below;
     }
-    if (r.node <= 0 || r.qsteps >= kNodes) {
-      if (r.qn > 0) { r.state = kLeafPending; r.pend = int(r.queue & 255u); break; }  // this lot's leaves first
-      r.state = kEnterLot;
-      continue;
-    }
-    r.qsteps++;
-    const int base = r.slot * kNodes;
-    // A node reached from its parent was tested against the same best a
-    // moment ago (the reference tests it again, with the same result); a node
-    // popped from the stack is tested again against the current best.
-    const bool near = r.fresh || nodeEntry(N, base + r.node, r.lr, r.inv0, r.best) < r.best;
-    r.fresh = 0;
-    if (near && r.node < kGroups) {
-      int left = r.node * 2, right = left + 1;
-      float ln = nodeEntry(N, base + left, r.lr, r.inv0, r.best), rn = nodeEntry(N, base + right, r.lr, r.inv0, r.best);
-      bool lh = ln < r.best, rh = rn < r.best;
-      r.fresh = lh || rh;
-      if (lh && rh) {
-        int next = ln < rn ? left : right, other = ln < rn ? right : left;
-        r.stack = (r.stack << 7) | (unsigned long long)other;
-        r.node = next;
-      } else if (lh) r.node = left;
-      else if (rh) r.node = right;
-      else r.node = popNode(r.stack);
-    } else {
-      if (near && r.node >= kGroups) {
-        r.queue |= unsigned(r.node - kGroups) << (8 * r.qn);
-        r.qn++;
-        r.node = popNode(r.stack);
-        if (r.qn == kSpec) { r.state = kLeafPending; r.pend = int(r.queue & 255u); break; }
-        continue;
-      }
-      r.node = popNode(r.stack);
+    r.leaves ^= cur;
+    const int leaf = __ffsll(cur) - 1;
+    if (!r.moved || nodeEntry(N, r.slot * kNodes + kGroups + leaf, r.lr, r.inv0, r.best) < r.best) {
+      r.pend = leaf;
+      r.state = kLeafPending;
+      return;
     }
   }
+}
+
+// Step the lane's DDA to the next lot whose root it enters before its best, or to its end.
+SD void coopEnterLot(CoopRay& r, const float* __restrict__ W, const float4* __restrict__ N, uint32_t o0, uint32_t o2) {
+#pragma unroll 1
+  while (r.state == kEnterLot) {
+    if (r.ddaSteps >= 160 || r.t > r.best || r.t > r.farT || r.t > kFar) { r.state = kDone; break; }
+    r.ddaSteps++;
+    r.slot = tableSlot(o0, o2, r.cx, r.cz);
+    r.lcx = r.cx; r.lcz = r.cz;
+    const float4 c = __ldg(reinterpret_cast<const float4*>(W + r.slot * kLotFloats) + 2);  // roofScale, turn, ox, oz
+    const int turn = int(c.y);
+    f3 cp = mk(float(r.cx) * kCell + c.z, 0.0f, float(r.cz) * kCell + c.w);
+    r.lr = toLot(r.ro - cp, turn);
+    r.ld = toLot(r.rd, turn);
+    r.inv0 = invDir(r.ld);
+    // the DDA steps to the next cell now; the reference does it after the
+    // lot's query, and the next test reads only t and the (later) best
+    if (r.tx < r.tz) { r.t = r.tx; r.tx += r.dx; r.cx += r.sx; } else { r.t = r.tz; r.tz += r.dz; r.cz += r.sz; }
+    if (nodeEntry(N, r.slot * kNodes + 1, r.lr, r.inv0, r.best) < r.best) r.state = kLotPending;
+  }
+}
+
+// The rays of `peer` lanes, all in the same lot, as one packet.  Warp-collective.
+SD Packet lotPacket(const CoopRay& r, bool peer, int src) {
+  const float big = 1e30f;
+  Packet k;
+  k.ro = mk(__shfl_sync(0xffffffffu, r.lr.x, src), __shfl_sync(0xffffffffu, r.lr.y, src),
+            __shfl_sync(0xffffffffu, r.lr.z, src));
+  k.lo = mk(warpMin(peer ? r.inv0.x : big), warpMin(peer ? r.inv0.y : big), warpMin(peer ? r.inv0.z : big));
+  k.hi = mk(warpMax(peer ? r.inv0.x : -big), warpMax(peer ? r.inv0.y : -big), warpMax(peer ? r.inv0.z : -big));
+  k.best = warpMax(peer ? r.best : 0.0f);
+  return k;
 }
 
 // Inverse of the turn-1 direction (ld.z, ld.y, -ld.x): a permutation of inv0
@@ -249,38 +301,6 @@ SD Feat winnerFeature(const GroupCache& c, const float* __restrict__ W, int slot
 constexpr int kRunsPerGroup = (kEntryRecords + kRun - 1) / kRun;
 // Shared memory of one warp: the records of the group it serves.
 struct WarpStage { StagedFeat feats[kEntryRecords]; };
-
-// The rays a warp serves together, as one packet: they leave one point (the
-// camera in the lot's frame) with inverse directions between lo and hi, and
-// none wants a hit beyond `best`.
-struct Packet { f3 ro, lo, hi; float best; };
-
-// Whether some ray of the packet may hit this record nearer than its own best.
-// A ray's slab times of an axis are linear in its inverse direction, so over the
-// packet they lie between the extremes of the four products of the box's two
-// planes with the interval's two ends; a record is out when the latest of the
-// axes' earliest entries is past the earliest of their latest exits, or past
-// every ray's best.  The latter holds for boxes (masonry relief included, inside the
-// pad) and prisms only: quadrics and foliage are bounded by the box test alone.
-// The 0.025 m pad covers every rounding of this test and of the exact one: at
-// |ro| <= 2,100 m (a visited lot is at most 2,000 m along a ray) they sum to
-// less than 0.001 m.
-SD bool packetMayHit(const StagedFeat& s, const Packet& k) {
-  const int shape = (s.packed & 255) - 1;
-  const bool odd = (s.packed >> 16) & 1, base = shape == 3 || shape == 4;  // these stand on p.y
-  const float hx = (odd ? s.hz : s.hx) + 0.025f, hz = (odd ? s.hx : s.hz) + 0.025f, hy = s.hy + 0.025f;
-  const float ax = s.px - hx - k.ro.x, bx = s.px + hx - k.ro.x;
-  const float ay = (base ? s.py - 0.025f : s.py - hy) - k.ro.y, by = s.py + hy - k.ro.y;
-  const float az = s.pz - hz - k.ro.z, bz = s.pz + hz - k.ro.z;
-  const float x0 = ax * k.lo.x, x1 = ax * k.hi.x, x2 = bx * k.lo.x, x3 = bx * k.hi.x;
-  const float y0 = ay * k.lo.y, y1 = ay * k.hi.y, y2 = by * k.lo.y, y3 = by * k.hi.y;
-  const float z0 = az * k.lo.z, z1 = az * k.hi.z, z2 = bz * k.lo.z, z3 = bz * k.hi.z;
-  const float in = fmaxf(fmaxf(fminf(fminf(x0, x1), fminf(x2, x3)), fminf(fminf(y0, y1), fminf(y2, y3))),
-                         fminf(fminf(z0, z1), fminf(z2, z3)));
-  const float out = fminf(fminf(fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)), fmaxf(fmaxf(y0, y1), fmaxf(y2, y3))),
-                          fmaxf(fmaxf(z0, z1), fmaxf(z2, z3)));
-  return in <= out && out >= 0.001f && (in <= k.best || !(shape == 0 || shape == 3));
-}
 
 // Group records shared by the warps of one block, for a trace with no
 // table-wide group cache (the drop-in entry point).  Write-once for the
@@ -331,19 +351,57 @@ SD void blockCachePut(BlockCache& bc, const WarpStage& ws, int key, int count) {
   if (lane == 0) bc.ready[e] = 1;
 }
 
-// Stage one group: its records from the group cache, or built by the grammar
-// (and stored when the cache gives an entry), and, where `boxes` is given, the
-// chunk boxes.  Warp-collective; returns the group's record count.
+// Build one group's records by the grammar, one feature a lane, storing them
+// (with the chunk boxes) when the cache gives an entry; `word` is the directory
+// word the caller read.  Warp-collective, out of line: the rare path of a warm
+// cache.  `boxes` may be null.
+static __device__ __noinline__ void buildGroup(const float* __restrict__ W, GroupCache cache, int key, int count,
+                                               uint32_t word, StagedFeat* feats, ChunkBox* boxes) {
+  const int lane = int(threadIdx.x & 31);
+  const int slot = key >> 6, g = key & 63;
+  const LotDesc L = loadLot(W, slot);
+  const int e = cacheClaim(cache, slot, g, word);  // -1: build without storing
+#pragma unroll 1
+  for (int base = 0; base < count; base += 32) {
+    const int j = base + lane;
+    f3 lo = mk(1e30f, 1e30f, 1e30f), hi = mk(-1e30f, -1e30f, -1e30f);
+    if (j < count) {
+      StagedFeat s;
+      stage(s, featureAtOOL(L, g, j));
+      if (e >= 0) entryRecords(cache, uint32_t(e))[j] = s;
+      feats[j] = s;
+      hitBox(unstage(s), lo, hi);
+    }
+    if (e < 0 && !boxes) continue;
+#pragma unroll
+    for (int o = 1; o < kRun; o <<= 1) {
+      lo = vmin(lo, mk(__shfl_xor_sync(0xffffffffu, lo.x, o), __shfl_xor_sync(0xffffffffu, lo.y, o),
+                       __shfl_xor_sync(0xffffffffu, lo.z, o)));
+      hi = vmax(hi, mk(__shfl_xor_sync(0xffffffffu, hi.x, o), __shfl_xor_sync(0xffffffffu, hi.y, o),
+                       __shfl_xor_sync(0xffffffffu, hi.z, o)));
+    }
+    if ((lane & (kRun - 1)) == 0 && j < count) {
+      if (boxes) boxes[j / kRun] = ChunkBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
+      if (e >= 0) {
+        float* bp = entryBoxes(cache, uint32_t(e)) + (j / kRun) * 6;
+        bp[0] = lo.x; bp[1] = lo.y; bp[2] = lo.z; bp[3] = hi.x; bp[4] = hi.y; bp[5] = hi.z;
+      }
+    }
+  }
+  if (e >= 0) cachePublish(cache, W, slot, g, count, e);
+}
+
+// Stage one group's records and chunk boxes, from the group cache or built.
+// Warp-collective; returns the group's record count.
 SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key, StagedFeat* feats, ChunkBox* boxes) {
   const int lane = int(threadIdx.x & 31);
   const int slot = key >> 6, g = key & 63;
   // the directory word, the lot row, the entry's tag and its records in as few
   // dependent round trips as possible: the records are loaded with the tag and
   // kept only if every tag word matches the slot's current descriptor (else a miss)
-  uint32_t word = cache.base ? __ldcg(cache.dir(slot, g)) : 0u;
-  const LotDesc L = loadLot(W, slot);
-  const int count = groupCount(L, g);
-  int e = cache.base ? usableEntry(cache, word) : -1;
+  const uint32_t word = cache.base ? __ldcg(cache.dir(slot, g)) : 0u;
+  const int count = groupCount(loadLot(W, slot), g);
+  const int e = cache.base ? usableEntry(cache, word) : -1;
   if (e >= 0) {
     bool same = true;
     if (lane < kEntryTagWords)
@@ -351,7 +409,7 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
     StagedFeat r0{}, r1{};
     if (lane < count) r0 = cacheRecord(cache, e, lane);
     if (lane + 32 < count) r1 = cacheRecord(cache, e, lane + 32);
-    const int runs = boxes ? (count + kRun - 1) / kRun : 0;
+    const int runs = (count + kRun - 1) / kRun;
     float2 ba{}, bb{}, bc{};
     if (lane < runs) {
       const float2* bp = reinterpret_cast<const float2*>(entryBoxes(cache, uint32_t(e)) + lane * 6);
@@ -361,43 +419,94 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
       if (lane < count) feats[lane] = r0;
       if (lane + 32 < count) feats[lane + 32] = r1;
       if (lane < runs) boxes[lane] = ChunkBox{{ba.x, ba.y, bb.x}, {bb.y, bc.x, bc.y}};
-    } else {
-      e = -1;
+      return count;
     }
   }
-  const bool cached = e >= 0;
-  if (!cached) e = cacheClaim(cache, slot, g, word);  // -1: build without storing
-  if (!cached) {
-#pragma unroll 1
-    for (int base = 0; base < count; base += 32) {
-      const int j = base + lane;
-      f3 lo = mk(1e30f, 1e30f, 1e30f), hi = mk(-1e30f, -1e30f, -1e30f);
-      if (j < count) {
-        StagedFeat s;
-        stage(s, featureAtOOL(L, g, j));
-        if (e >= 0) entryRecords(cache, uint32_t(e))[j] = s;
-        feats[j] = s;
-        hitBox(unstage(s), lo, hi);
-      }
-      if (e < 0 && !boxes) continue;
-#pragma unroll
-      for (int o = 1; o < kRun; o <<= 1) {
-        lo = vmin(lo, mk(__shfl_xor_sync(0xffffffffu, lo.x, o), __shfl_xor_sync(0xffffffffu, lo.y, o),
-                         __shfl_xor_sync(0xffffffffu, lo.z, o)));
-        hi = vmax(hi, mk(__shfl_xor_sync(0xffffffffu, hi.x, o), __shfl_xor_sync(0xffffffffu, hi.y, o),
-                         __shfl_xor_sync(0xffffffffu, hi.z, o)));
-      }
-      if ((lane & (kRun - 1)) == 0 && j < count) {
-        if (boxes) boxes[j / kRun] = ChunkBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
-        if (e >= 0) {
-          float* bp = entryBoxes(cache, uint32_t(e)) + (j / kRun) * 6;
-          bp[0] = lo.x; bp[1] = lo.y; bp[2] = lo.z; bp[3] = hi.x; bp[4] = hi.y; bp[5] = hi.z;
-        }
-      }
-    }
-  }
-  if (!cached && e >= 0) cachePublish(cache, W, slot, g, count, e);
+  buildGroup(W, cache, key, count, word, feats, boxes);
   return count;
+}
+
+// Records lane and lane + 32 of a group: from its cache entry, whose tag and
+// records are read in one round trip and kept if the tag holds the slot's
+// current descriptor words, else from the block's table or built.
+// Warp-collective; returns the record count.
+template <bool kBlockCache>
+SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockCache* bc, int key, WarpStage& ws,
+                    StagedFeat& r0, StagedFeat& r1) {
+  const int lane = int(threadIdx.x & 31);
+  const int slot = key >> 6, g = key & 63;
+  const StagedFeat* feats = ws.feats;
+  uint32_t word = 0u;
+  int count, held = -1;
+  if constexpr (kBlockCache) {
+    held = blockCacheFind(*bc, key);
+    if (held >= 0) {  // built earlier by a warp of this block
+      count = bc->count[held];
+      feats = bc->feats[held];
+    }
+  } else if (cache.base) {
+    const uint32_t row = lane < 9 ? __float_as_uint(__ldg(W + slot * kLotFloats + lane)) : 0u;
+    word = __ldcg(cache.dir(slot, g));
+    const int e = usableEntry(cache, word);
+    if (e >= 0) {
+      const uint32_t tag = lane < kEntryTagWords ? __ldg(entryTag(cache, uint32_t(e)) + lane) : 0u;
+      r0 = cacheRecord(cache, e, lane);
+      r1 = cacheRecord(cache, e, min(lane + 32, kEntryRecords - 1));
+      const bool same = lane < 9 ? tag == row : lane != 9 || tag == uint32_t(g);
+      if (__all_sync(0xffffffffu, same)) return int(__shfl_sync(0xffffffffu, tag, 10));
+    }
+  }
+  if (held < 0) {
+    count = groupCount(loadLot(W, slot), g);
+    buildGroup(W, cache, key, count, word, ws.feats, nullptr);
+    __syncwarp();
+    if constexpr (kBlockCache) blockCachePut(*bc, ws, key, count);
+  }
+  r0 = feats[lane];
+  r1 = feats[min(lane + 32, kEntryRecords - 1)];
+  __syncwarp();
+  return count;
+}
+
+// Advance every lane until it has a leaf to evaluate or is done.  Warp-collective.
+SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __restrict__ N, uint32_t o0, uint32_t o2) {
+  const int lane = int(threadIdx.x & 31);
+#pragma unroll 1
+  for (;;) {
+    coopEnterLot(r, W, N, o0, o2);
+    unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
+    if (!lots) return;
+#pragma unroll 1
+    while (lots) {
+      const int src = __ffs(lots) - 1, slot = __shfl_sync(0xffffffffu, r.slot, src);
+      const bool peer = r.state == kLotPending && r.slot == slot;
+      lots &= ~__ballot_sync(0xffffffffu, peer);
+      // lanes are leaves: which of the lot's 64 can any peer's ray enter
+      const float4* leaf = N + 2 * (slot * kNodes + kGroups + lane);
+      const float4 a0 = __ldg(leaf), b0 = __ldg(leaf + 1), a1 = __ldg(leaf + 64), b1 = __ldg(leaf + 65);
+      const Packet pk = lotPacket(r, peer, src);
+      unsigned m0 = __ballot_sync(0xffffffffu, a0.w > 0.5f && packetMayEnter(a0, b0, pk));
+      unsigned m1 = __ballot_sync(0xffffffffu, a1.w > 0.5f && packetMayEnter(a1, b1, pk));
+      if (peer) {
+        const int base = slot * kNodes + kGroups;
+        unsigned lo = 0u, hi = 0u;
+#pragma unroll 1
+        for (; m0; m0 &= m0 - 1u) {
+          const int k = __ffs(m0) - 1;
+          if (nodeEntry(N, base + k, r.lr, r.inv0, r.best) < r.best) lo |= 1u << k;
+        }
+#pragma unroll 1
+        for (; m1; m1 &= m1 - 1u) {
+          const int k = __ffs(m1) - 1;
+          if (nodeEntry(N, base + 32 + k, r.lr, r.inv0, r.best) < r.best) hi |= 1u << k;
+        }
+        r.leaves = (unsigned long long)hi << 32 | lo;
+        orderLeaves(r, N);
+        nextLeaf(r, N);
+      }
+      __syncwarp();
+    }
+  }
 }
 
 // The whole warp traces its 32 rays.  Every lane of the warp must call this
@@ -424,35 +533,15 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
       const int key = __shfl_sync(0xffffffffu, myKey, __ffs(pending) - 1);
       const bool peer = r.state == kLeafPending && myKey == key;
       const unsigned peers = __ballot_sync(0xffffffffu, peer);
-      int count;
-      const StagedFeat* feats = ws.feats;
-      if constexpr (kBlockCache) {
-        const int e = blockCacheFind(*bc, key);
-        if (e >= 0) {  // built earlier by a warp of this block
-          count = bc->count[e];
-          feats = bc->feats[e];
-          __syncwarp();
-        } else {
-          count = stageGroup(W, cache, key, ws.feats, nullptr);
-          __syncwarp();
-          blockCachePut(*bc, ws, key, count);
-        }
-      } else {
-        count = stageGroup(W, cache, key, ws.feats, nullptr);
-        __syncwarp();
-      }
-      // lanes are records: which of them can any peer's ray hit
-      const float big = 1e30f;
-      Packet pk;
-      const int src = __ffs(peers) - 1;
-      pk.ro = mk(__shfl_sync(0xffffffffu, r.lr.x, src), __shfl_sync(0xffffffffu, r.lr.y, src),
-                 __shfl_sync(0xffffffffu, r.lr.z, src));
-      pk.lo = mk(warpMin(peer ? r.inv0.x : big), warpMin(peer ? r.inv0.y : big), warpMin(peer ? r.inv0.z : big));
-      pk.hi = mk(warpMax(peer ? r.inv0.x : -big), warpMax(peer ? r.inv0.y : -big), warpMax(peer ? r.inv0.z : -big));
-      pk.best = warpMax(peer ? r.best : 0.0f);
-      const unsigned m0 = __ballot_sync(0xffffffffu, lane < count && packetMayHit(feats[lane], pk));
-      const unsigned m1 =
-          count <= 32 ? 0u : __ballot_sync(0xffffffffu, lane + 32 < count && packetMayHit(feats[lane + 32], pk));
+      // lanes are records: which of the group's can any peer's ray hit
+      StagedFeat r0, r1;
+      const int count = groupRecords<kBlockCache>(W, cache, bc, key, ws, r0, r1);
+      const Packet pk = lotPacket(r, peer, __ffs(peers) - 1);
+      const unsigned m0 = __ballot_sync(0xffffffffu, lane < count && packetMayHit(r0, pk));
+      const unsigned m1 = count <= 32 ? 0u : __ballot_sync(0xffffffffu, lane + 32 < count && packetMayHit(r1, pk));
+      if ((m0 >> lane) & 1u) ws.feats[lane] = r0;
+      if ((m1 >> lane) & 1u) ws.feats[lane + 32] = r1;
+      __syncwarp();
       if (peer) {
         // those records in index order: the first feature wins ties
         const int g = r.pend;
@@ -461,7 +550,7 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
         while (mlo | mhi) {
           const int k = mlo ? __ffs(mlo) - 1 : __ffs(mhi) + 31;
           if (mlo) mlo &= mlo - 1u; else mhi &= mhi - 1u;
-          const Feat f = unstage(feats[k]);
+          const Feat f = unstage(ws.feats[k]);
           const bool odd = f.turn % 2 == 1;
           const f3 inv = odd ? inv1Of(r) : r.inv0, p = intoFeature(r.lr - f.p, f.turn);
           const Span rg = featureSlab(f, p, inv);
@@ -483,19 +572,10 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
           }
           if (th > 0.001f && th < r.best) {
             r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
+            r.moved = true;
           }
         }
-        // the next queued leaf that can still win (its node tested against
-        // the best just found, as the reference tests it when it gets there)
-        r.queue >>= 8;
-        r.qn--;
-#pragma unroll 1
-        while (r.qn > 0 && !(nodeEntry(N, r.slot * kNodes + kGroups + int(r.queue & 255u), r.lr, r.inv0, r.best) < r.best)) {
-          r.queue >>= 8;
-          r.qn--;
-        }
-        if (r.qn > 0) r.pend = int(r.queue & 255u);
-        else r.state = kInLot;  // the walk goes on from where it stopped
+        nextLeaf(r, N);
       }
       __syncwarp();
       pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);

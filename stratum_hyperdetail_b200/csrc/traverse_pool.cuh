@@ -152,21 +152,11 @@ SD TraceResult tracePooled(PoolShared<P>& sh, const stratum_view* __restrict__ V
         if (sh.best[tid] < r.best) {  // the served group holds a nearer feature
           r.best = sh.best[tid];
           r.fid = sh.fid[tid];
+          r.moved = true;
           r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
         }
-        r.queue >>= 8;
-        r.qn--;
-#pragma unroll 1
-        while (r.qn > 0 && !(nodeEntry(N, r.slot * kNodes + kGroups + int(r.queue & 255u), r.lr, r.inv0, r.best) < r.best)) {
-          r.queue >>= 8;
-          r.qn--;
-        }
-        if (r.qn > 0) {
-          r.pend = int(r.queue & 255u);
-        } else {
-          r.state = kInLot;  // the walk goes on from where it stopped
-          pend = false;
-        }
+        nextLeaf(r, N);
+        pend = r.state == kLeafPending;
         sh.key[tid] = pend ? poolKey(view, r.slot, r.pend) : -1;
       }
       if (!__syncthreads_or(pend)) break;
