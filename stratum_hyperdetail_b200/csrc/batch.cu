@@ -150,8 +150,6 @@ SD void retire(uint32_t* next, uint32_t* done, int threads) {
 // SM (128 registers, a few bytes of spills): the six-view 1600x900 trace 4-5 %
 // faster than at 640 (96 registers, 88/136 bytes of spills), every pose faster;
 // 768 (80 registers, heavy spills) is slower still.
-// The warp-cooperative traversal (traverse_coop.cuh) unless built with
-// STRATUM_BATCH_PER_LANE (each lane walks its own ray, as the drop-in kernel).
 #ifndef STRATUM_TRACE_OCC
 #define STRATUM_TRACE_OCC 512
 #endif
@@ -177,16 +175,10 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
       const Camera cam = S->view[v].cam;
       const uint32_t o0 = S->view[v].o[0], o2 = S->view[v].o[2];
       f3 rd = primaryDir(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
-#ifdef STRATUM_BATCH_PER_LANE
-      if (!inFrame) continue;
-      TraceResult r = traceRay(V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2, cam.pos, rd,
-                               1.08f / float(H));
-#else
       TraceResult r = traceWarp(V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2, cam.pos, rd,
                                 1.08f / float(H), inFrame, reinterpret_cast<WarpStage*>(stageBytes)[warp],
                                 groupCache(V[v].Groups));
       if (!inFrame) continue;
-#endif
       storeTrace(V[v].Hit, V[v].Surface, size_t(y) * W + x, r);
     }
   }

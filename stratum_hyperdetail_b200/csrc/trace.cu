@@ -11,9 +11,7 @@
 // has built reads it from there (neighbouring tiles reach the same groups: on
 // the bench poses a 16x16 block needs 6-9x fewer group builds than its warps
 // would alone).  Each ray still visits its leaves in the reference's order with
-// the same running best, so Hit and Surface equal the per-thread traversal
-// (traverse.cuh) bit for bit; building with STRATUM_DROPIN_PER_LANE selects that
-// per-thread form instead.
+// the same running best, so Hit and Surface equal the reference's bit for bit.
 //
 // The reference's 64-row strips leave each launch a tail of partly idle SMs:
 // six 1600x900 views in 15 strips each trace in 24.4 ms, in one call per view
@@ -69,16 +67,10 @@ __global__ void __launch_bounds__(kDropInThreads, STRATUM_DROPIN_BLOCKS)
   const int y = rowStart + int(blockIdx.y) * kDropInH + (warp / kDropInTilesX) * 4 + (lane >> 3);
   const bool active = x < width && y < height && y < rowStart + rowCount;
   const f3 rd = primaryDir(cam, active ? x : 0, active ? y : 0, width, height);
-#ifdef STRATUM_DROPIN_PER_LANE
-  if (!active) return;
-  const TraceResult r = traceRay(W, reinterpret_cast<const float4*>(N), org[0], org[2], cam.pos, rd,
-                                 1.08f / float(height));
-#else
   const TraceResult r = traceWarp<true>(W, reinterpret_cast<const float4*>(N), org[0], org[2], cam.pos, rd,
                                         1.08f / float(height), active, sh.stage[warp], groupCache(nullptr),
                                         &sh.cache);
   if (!active) return;
-#endif
   storeTrace(Hit, Surface, size_t(y) * width + x, r);
 }
 
