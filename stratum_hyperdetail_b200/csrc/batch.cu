@@ -95,20 +95,24 @@ __global__ void cacheInitK(uint32_t* base, uint32_t entries) {
   h->next = 0u; h->capacity = entries; h->resets = 0u; h->fills = 0u; h->launches = 0u; h->resetAt = 0u;
 }
 
-__global__ void prologueK(stratum_view* V, int n, int order, BatchScratch* S) {
-  if (threadIdx.x == 0) {
-    int base = 0;
-    for (int v = 0; v < n; v++) {
-      V[v].tileBase = base;
-      V[v].tilesX = (V[v].width + kTileW - 1) / kTileW;
-      // a view with no pixels owns no tiles (and is never looked up)
-      if (V[v].width > 0 && V[v].height > 0) base += tileCount(V[v].width, V[v].height, order);
-    }
-    S->counters[kTotalTiles] = uint32_t(base);
-    S->taps = makeTaps();
-  }
+// `bandTiles`: band tiles to give out over all views: twice the warps the device
+// holds.  Warm trace of one 640x360 view, street / rooftop / aerial / canal / avenue:
+// no band 417 / 486 / 637 / 399 / 460 us, once the warps 363 / 484 / 629 / 359 / 285,
+// twice 309 / 355 / 634 / 248 / 291, four times 324 / 377 / 723 / 262 / 310.  A view
+// of a large batch still gets one tile row.
+__global__ void prologueK(stratum_view* V, int n, int order, int bandTiles, BatchScratch* S) {
   for (int v = int(threadIdx.x); v < n; v += int(blockDim.x)) {
-    S->view[v] = makeFrame(V[v].C, V[v].Origin);
+    S->view[v].frame = makeFrame(V[v].C, V[v].Origin);
+    const int W = V[v].width, H = V[v].height;
+    V[v].tilesX = (W + kTileW - 1) / kTileW;
+    Band& b = S->view[v].band;
+    b.horizon = b.row0 = b.row1 = 0;
+    if (W > 0 && H > 0) {
+      const int rows = (H + kTileH - 1) / kTileH, want = max(1, bandTiles / n / (V[v].tilesX * kTileH)), band = min(want, rows);
+      b.horizon = horizonRow(S->view[v].frame.cam, H);
+      b.row0 = min(max(b.horizon / kTileH - band / 2, 0), rows - band);
+      b.row1 = b.row0 + band;
+    }
     if (V[v].Groups) {  // this launch's epoch; a full cache starts again now and then
       GroupCacheHeader* h = reinterpret_cast<GroupCacheHeader*>(V[v].Groups);
       h->launches++;
@@ -119,6 +123,22 @@ __global__ void prologueK(stratum_view* V, int n, int order, BatchScratch* S) {
       }
     }
   }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int base = 0, band = 0;
+    for (int v = 0; v < n; v++) {
+      V[v].tileBase = base;
+      S->view[v].band.base = band;
+      // a view with no pixels owns no tiles (and is never looked up)
+      if (V[v].width > 0 && V[v].height > 0) {
+        base += tileCount(V[v].width, V[v].height, order);
+        band += bandCount(S->view[v].band, V[v].tilesX, V[v].height);
+      }
+    }
+    S->counters[kTotalTiles] = uint32_t(base);
+    S->counters[kBandTiles] = uint32_t(band);
+    S->taps = makeTaps();
+  }
 }
 
 // Last view whose first tile is <= tile (binary search; warp-uniform).
@@ -127,6 +147,15 @@ SD int viewOf(const stratum_view* __restrict__ V, int n, int tile) {
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
     if (V[mid].tileBase <= tile) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+SD int bandViewOf(const BatchScratch* S, int n, int tile) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (S->view[mid].band.base <= tile) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -158,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
     traceViewsK(const stratum_view* __restrict__ V, int n, int grab, int order, BatchScratch* S) {
   extern __shared__ __align__(16) unsigned char stageBytes[];  // THREADS / 32 WarpStage
   const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-  const int total = int(S->counters[kTotalTiles]);
+  const int bands = int(S->counters[kBandTiles]), total = bands + int(S->counters[kTotalTiles]);
 #pragma unroll 1
   for (;;) {
     const int t0 = claim(&S->counters[kTraceNext], grab);
@@ -166,14 +195,28 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
     const int t1 = min(t0 + grab, total);
 #pragma unroll 1
     for (int tile = t0; tile < t1; tile++) {
-      const int v = viewOf(V, n, tile);
+      const int v = tile < bands ? bandViewOf(S, n, tile) : viewOf(V, n, tile - bands);
       const int W = V[v].width, H = V[v].height;
-      int tx, ty;
-      if (!tileCoord(tile - V[v].tileBase, V[v].tilesX, (H + kTileH - 1) / kTileH, order, tx, ty)) continue;
-      const int x = tx * kTileW + (lane & 7), y = ty * kTileH + (lane >> 3);
-      const bool inFrame = x < W && y < H;
-      const Camera cam = S->view[v].cam;
-      const uint32_t o0 = S->view[v].o[0], o2 = S->view[v].o[2];
+      const Band band = S->view[v].band;
+      int x, y;
+      bool inFrame;
+      if (tile < bands) {
+        const int local = tile - band.base, first = band.row0 * kTileH, rows = min(band.row1 * kTileH, H) - first;
+        x = (local % V[v].tilesX) * kTileW + lane;
+        y = first + nearRow(local / V[v].tilesX, min(max(band.horizon - first, 0), rows - 1), rows);
+        inFrame = lane < kTileW && x < W;
+      } else {
+        int tx, ty;
+        if (!tileCoord(tile - bands - V[v].tileBase, V[v].tilesX, (H + kTileH - 1) / kTileH, order, tx, ty,
+                       band.horizon / kTileH) ||
+            (ty >= band.row0 && ty < band.row1))
+          continue;
+        x = tx * kTileW + (lane & 7);
+        y = ty * kTileH + (lane >> 3);
+        inFrame = x < W && y < H;
+      }
+      const Camera cam = S->view[v].frame.cam;
+      const uint32_t o0 = S->view[v].frame.o[0], o2 = S->view[v].frame.o[2];
       f3 rd = primaryDir(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
       TraceResult r = traceWarp(V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2, cam.pos, rd,
                                 1.08f / float(H), inFrame, reinterpret_cast<WarpStage*>(stageBytes)[warp],
@@ -214,8 +257,8 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
     }
     const int x = tx * kTileW + (lane & 7), y = ty * kTileH + (lane >> 3);
     const bool inFrame = ok && x < W && y < H;
-    const Camera cam = S->view[v].cam;
-    const uint32_t o0 = S->view[v].o[0], o2 = S->view[v].o[2];
+    const Camera cam = S->view[v].frame.cam;
+    const uint32_t o0 = S->view[v].frame.o[0], o2 = S->view[v].frame.o[2];
     const f3 rd = primaryDir(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
     const TraceResult r = tracePooled<P>(sh, V, v, V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2,
                                          cam.pos, rd, 1.08f / float(H), inFrame);
@@ -247,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_SHADE_OCC / THREADS) shadeVie
       if (!tileCoord(tile - V[v].tileBase, V[v].tilesX, (H + kTileH - 1) / kTileH, order, tx, ty)) continue;
       const int x = tx * kTileW + (lane & 7), y = ty * kTileH + (lane >> 3);
       if (x >= W || y >= H) continue;
-      const FrameConst F = S->view[v];
+      const FrameConst F = S->view[v].frame;
       const size_t b = size_t(y) * W + x;
       const float4* hit = reinterpret_cast<const float4*>(V[v].Hit);
       const float4* surf = reinterpret_cast<const float4*>(V[v].Surface);
@@ -294,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_SHADE_OCC / THREADS) lightVie
       const size_t b = size_t(y) * W + x;
       const float4 h4 = reinterpret_cast<const float4*>(V[v].Hit)[b];
       if (int(h4.y) == kSkyId) continue;
-      const FrameConst F = S->view[v];
+      const FrameConst F = S->view[v].frame;
       const f3 rd = primaryDir(F.cam, x, y, W, H);
       float4* lin = reinterpret_cast<float4*>(V[v].Linear) + b;
       const float4 a = *lin;
@@ -325,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_RESOLVE_OCC / THREADS) resolv
       if (!tileCoord(tile - V[v].tileBase, V[v].tilesX, (H + kTileH - 1) / kTileH, order, tx, ty)) continue;
       const int x = tx * kTileW + (lane & 7), y = ty * kTileH + (lane >> 3);
       if (x >= W || y >= H) continue;
-      const FrameConst F = S->view[v];
+      const FrameConst F = S->view[v].frame;
       const size_t b = size_t(y) * W + x;
       const float4 l = reinterpret_cast<const float4*>(V[v].Linear)[b];
       resolvePixel(mk(l.x, l.y, l.z), reinterpret_cast<float4*>(V[v].History), V[v].Pixels, F, S->taps,
@@ -357,7 +400,7 @@ constexpr int kGridDevices = 64;
 struct PersistentGrids { int trace, pooled, shade, light, resolve; };
 
 template <int T>
-int launchParts(const stratum_view* V, int n, const stratum_tune& t, BatchScratch* S, cudaStream_t s, int parts) {
+int launchParts(stratum_view* V, int n, const stratum_tune& t, BatchScratch* S, cudaStream_t s, int parts) {
   static std::once_flag once[kGridDevices];
   static PersistentGrids grids[kGridDevices];
   int dev = 0;
@@ -375,6 +418,10 @@ int launchParts(const stratum_view* V, int n, const stratum_tune& t, BatchScratc
   });
   const PersistentGrids& g = grids[dev];
   const int order = t.order & 1;  // tile order; bit 1 selects the block-pooled trace
+  if (parts & kTrace) {
+    prologueK<<<1, 256, 0, s>>>(V, n, order, 2 * g.trace * (T / 32), S);
+    cacheResetK<<<dim3(64, n), 256, 0, s>>>(V, n);
+  }
   if ((parts & kTrace) && (t.order & 2))
     tracePooledK<T><<<g.pooled, T, sizeof(PoolShared<T / 32>), s>>>(V, n, order, S);
   else if (parts & kTrace)
@@ -397,10 +444,6 @@ int render(stratum_view* V, int n, void* scratch, unsigned long long bytes, cons
   stratum_tune t = tune ? *tune : stratum_tune{128, 1, 1};
   if (!tuneOk(t)) return STRATUM_EINVAL;
   BatchScratch* S = static_cast<BatchScratch*>(scratch);
-  if (parts & kTrace) {
-    prologueK<<<1, 256, 0, s>>>(V, n, t.order & 1, S);
-    cacheResetK<<<dim3(64, n), 256, 0, s>>>(V, n);
-  }
   if (t.threads == 64) return launchParts<64>(V, n, t, S, s, parts);
   if (t.threads == 256) return launchParts<256>(V, n, t, S, s, parts);
   return launchParts<128>(V, n, t, S, s, parts);

@@ -19,15 +19,30 @@ enum : int {
   kResolveDone = 6,
   kLightNext = 7,
   kLightDone = 8,
+  kBandTiles = 9,   // band tiles over all views (written by the prologue)
   kCounters = 16
+};
+// The trace draws a band of tile rows around the horizon first, in tiles one
+// pixel high, then everything else in whole tiles, nearest the horizon first.
+// A ray near the horizon crosses the most lots: the slowest tiles took 1 ms where
+// the mean took 25 us, so a frame waited for the few that were claimed late, and
+// a frame of fewer tiles than the device holds warps waited for its slowest tile.
+struct Band {
+  int base;        // first of the view's band tiles
+  int row0, row1;  // the band's tile rows
+  int horizon;     // pixel row of the horizon, inside the frame
+};
+struct ViewFrame {
+  FrameConst frame;
+  Band band;
 };
 struct BatchScratch {
   uint32_t counters[kCounters];
   ResolveTaps taps;
-  FrameConst view[1];  // n entries
+  ViewFrame view[1];  // n entries
 };
 inline size_t batchScratchBytes(int views) {
-  return sizeof(BatchScratch) + size_t(views > 1 ? views - 1 : 0) * sizeof(FrameConst);
+  return sizeof(BatchScratch) + size_t(views > 1 ? views - 1 : 0) * sizeof(ViewFrame);
 }
 
 // Tile count of a view under an order: row-major tiles, or whole 4x4-tile
@@ -37,16 +52,37 @@ SD int tileCount(int width, int height, int order) {
   if (order == 1) return ((tx + 3) / 4) * ((ty + 3) / 4) * 16;
   return tx * ty;
 }
-SD bool tileCoord(int local, int tilesX, int tilesY, int order, int& tx, int& ty) {
+// Rows in the order of their distance from row `h` (0 <= k, h < rows): h, then
+// its neighbours on either side by turns, then what is left of the longer side.
+HD int nearRow(int k, int h, int rows) {
+  const int side = h < rows - 1 - h ? h : rows - 1 - h;
+  if (k <= 2 * side) return (k & 1) ? h + (k + 1) / 2 : h - k / 2;
+  return side == h ? k : rows - 1 - k;
+}
+// The pixel row the camera's horizon falls on, kept inside the frame.
+SD int horizonRow(const Camera& c, int height) {
+  const float sy = -c.fwd.y / c.up.y, y = 0.5f * float(height) - 0.5f - c.jy - sy * float(height) / 1.08f;
+  return int(fminf(fmaxf(y, 0.0f), float(height - 1)));  // NaN (looking straight down): 0
+}
+
+// Tile `local` of a view: row-major, or super-tile rows of Morton-ordered
+// super-tiles; with `first` >= 0 the (super-)rows in the order of their distance
+// from tile row `first`.
+SD bool tileCoord(int local, int tilesX, int tilesY, int order, int& tx, int& ty, int first = -1) {
   if (order == 1) {
-    int st = local >> 4, w = local & 15, superX = (tilesX + 3) / 4;
+    int st = local >> 4, w = local & 15, superX = (tilesX + 3) / 4, row = st / superX;
+    if (first >= 0) row = nearRow(row, first / 4, (tilesY + 3) / 4);
     tx = (st % superX) * 4 + ((w & 1) | ((w >> 1) & 2));
-    ty = (st / superX) * 4 + (((w >> 1) & 1) | ((w >> 2) & 2));
+    ty = row * 4 + (((w >> 1) & 1) | ((w >> 2) & 2));
   } else {
     tx = local % tilesX;
     ty = local / tilesX;
+    if (first >= 0) ty = nearRow(ty, first, tilesY);
   }
   return tx < tilesX && ty < tilesY;
+}
+SD int bandCount(const Band& b, int tilesX, int height) {
+  return (min(b.row1 * kTileH, height) - b.row0 * kTileH) * tilesX;
 }
 
 }  // namespace st

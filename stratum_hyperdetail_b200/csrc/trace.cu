@@ -22,6 +22,7 @@
 // safe only when the preceding kernel is known to be another strip.
 #include <mutex>
 
+#include "batch.cuh"
 #include "common_api.cuh"
 #include "traverse_coop.cuh"
 
@@ -48,10 +49,13 @@ struct DropInShared {
   BlockCache cache;
 };
 
+// `bandRows` block rows nearest the horizon are drawn first, each by four blocks
+// whose warps take tiles one pixel high (see Band in batch.cuh), then the others,
+// nearest the horizon first.
 __global__ void __launch_bounds__(kDropInThreads, STRATUM_DROPIN_BLOCKS)
     tracePrimaryK(const float* __restrict__ W, const float* __restrict__ N, const uint32_t* __restrict__ O,
                   const float* __restrict__ C, float* Hit, float* Surface, int width, int height, int rowStart,
-                  int rowCount) {
+                  int rowCount, int blocksX, int bandRows) {
   extern __shared__ __align__(16) unsigned char dropInBytes[];
   DropInShared& sh = *reinterpret_cast<DropInShared*>(dropInBytes);
   __shared__ Camera cam;
@@ -63,9 +67,27 @@ __global__ void __launch_bounds__(kDropInThreads, STRATUM_DROPIN_BLOCKS)
   blockCacheInit(sh.cache);
   __syncthreads();
   const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-  const int x = int(blockIdx.x) * kDropInW + (warp % kDropInTilesX) * 8 + (lane & 7);
-  const int y = rowStart + int(blockIdx.y) * kDropInH + (warp / kDropInTilesX) * 4 + (lane >> 3);
-  const bool active = x < width && y < height && y < rowStart + rowCount;
+  const int strip = min(rowCount, height - rowStart), rows = (strip + kDropInH - 1) / kDropInH;
+  const int horizon = min(max(horizonRow(cam, height) - rowStart, 0), strip - 1), mid = horizon / kDropInH;
+  const int row0 = min(max(mid - bandRows / 2, 0), rows - bandRows);  // of the band
+  const int blockRow = int(blockIdx.x) / blocksX, blockX = int(blockIdx.x) % blocksX;
+  const int tileX = blockX * kDropInW + (warp % kDropInTilesX) * 8;
+  int x, y;
+  bool mine;
+  if (blockRow < 4 * bandRows) {
+    x = tileX + lane;
+    y = row0 * kDropInH + nearRow(blockRow, min(horizon / 4 - row0 * (kDropInH / 4), 4 * bandRows - 1), 4 * bandRows) * 4 +
+        warp / kDropInTilesX;
+    mine = lane < 8;
+  } else {
+    const int row = nearRow(blockRow - 4 * bandRows, mid, rows);
+    if (row >= row0 && row < row0 + bandRows) return;  // uniform over the block
+    x = tileX + (lane & 7);
+    y = row * kDropInH + (warp / kDropInTilesX) * 4 + (lane >> 3);
+    mine = true;
+  }
+  const bool active = mine && x < width && y < strip;
+  y += rowStart;
   const f3 rd = primaryDir(cam, active ? x : 0, active ? y : 0, width, height);
   const TraceResult r = traceWarp<true>(W, reinterpret_cast<const float4*>(N), org[0], org[2], cam.pos, rd,
                                         1.08f / float(height), active, sh.stage[warp], groupCache(nullptr),
@@ -80,6 +102,7 @@ using namespace st;
 
 namespace {
 constexpr int kSmemDevices = 64;
+static_assert(kDropInTilesY == 4 && kDropInH == 16, "a band block is a quarter of a block high");
 }
 
 extern "C" int stratum_tracePrimary(const float* World, const float* Nodes, const unsigned* Origin, const float* C,
@@ -90,13 +113,25 @@ extern "C" int stratum_tracePrimary(const float* World, const float* Nodes, cons
   int rows = rowCount < height - rowStart ? rowCount : height - rowStart;
   if (rows <= 0) return STRATUM_OK;
   static std::once_flag once[kSmemDevices];
+  static int resident[kSmemDevices];  // blocks the device holds
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kSmemDevices) return STRATUM_EINVAL;
-  std::call_once(once[dev], [] {
+  std::call_once(once[dev], [dev] {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaFuncSetAttribute(tracePrimaryK, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(DropInShared)));
+    resident[dev] = sms * STRATUM_DROPIN_BLOCKS;
   });
-  dim3 grid((width + kDropInW - 1) / kDropInW, (rows + kDropInH - 1) / kDropInH);
-  tracePrimaryK<<<grid, kDropInThreads, sizeof(DropInShared), asStream(stream)>>>(
-      World, Nodes, static_cast<const uint32_t*>(Origin), C, Hit, Surface, width, height, rowStart, rowCount);
+  // Band rows: up to twice the blocks the device holds in quarter blocks, but at
+  // most a sixth of a frame that fills the device by itself (a band row takes about
+  // two rows' time; a 64-row strip gets none).  One call, us, without / with: 320x180
+  // street 357 / 241, aerial 745 / 640; 640x360 street 535 / 360, canal 446 / 264;
+  // 1600x900 street 880 / 633, avenue 976 / 755, rooftop 860 / 950.
+  const int blocksX = (width + kDropInW - 1) / kDropInW, blockRows = (rows + kDropInH - 1) / kDropInH;
+  const int most = blocksX * blockRows <= resident[dev] ? blockRows : blockRows / 6;
+  const int want = (2 * resident[dev] - 1) / (4 * blocksX) + 1, bandRows = want < most ? want : most;
+  tracePrimaryK<<<blocksX * (blockRows + 4 * bandRows), kDropInThreads, sizeof(DropInShared), asStream(stream)>>>(
+      World, Nodes, static_cast<const uint32_t*>(Origin), C, Hit, Surface, width, height, rowStart, rowCount, blocksX,
+      bandRows);
   return launchStatus();
 }

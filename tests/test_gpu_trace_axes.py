@@ -48,3 +48,26 @@ def test_axis_aligned_packets(cuda, oracle, yaw, pitch, height):
             v.History.zero_()
             b.frame()
             check(f"{w}x{h} batched {again}", host_frame(v), want, second)
+
+
+@pytest.mark.parametrize("w,h,pitch", [(320, 180, 0.0), (640, 360, 0.9), (641, 363, -0.9), (1283, 121, -0.05), (5, 700, 0.02)])
+def test_band_and_strips_draw_every_pixel_alike(cuda, w, h, pitch):
+    """The horizon inside, above and below the frame, bands of none, some and all
+    of its rows: whole frame, 64-row strips (no band) and batched, bit for bit."""
+    from stratum_hyperdetail_b200.batch import Batch
+    from stratum_hyperdetail_b200.views import View
+    v = View(w, h)
+    v.set_pose(99, (3, 0, 4, 0), (17.0, 25.0, 3.0), 0.4, pitch)
+    kept = None
+    b = Batch([v], (64, 2, 0))
+    for draw in (v.frame, v.frame_parts, b.frame):
+        v.C[19] = 0.0
+        for t in (v.Hit, v.Surface, v.Linear, v.History, v.Pixels):
+            t.zero_()
+        draw()
+        got = host_frame(v)
+        if kept is None:
+            kept = got
+            assert (got["Hit"].reshape(-1, 4)[:, 0] > 0).all()  # every pixel was written
+        for name in kept:
+            assert np.array_equal(kept[name].view(np.uint32), got[name].view(np.uint32)), (draw, name)
