@@ -193,8 +193,7 @@ typedef struct stratum_view {
  * against the table's current descriptor rows, so the cache never needs
  * invalidating when the table is refreshed (by any entry point); a full cache
  * keeps serving its groups and is emptied at most every 8 batched frames.  A trace launch uses the
- * groups filled by earlier launches (the first frame of a view fills, the
- * following ones reuse; at most 16,777,214 entries).  Results are identical
+ * groups filled by earlier launches and by itself (at most 16,777,214 entries).  Results are identical
  * with and without a cache.  Initialise once before use (zeroes the directory,
  * sets the capacity); a zero-filled buffer is a cache of capacity 0. */
 unsigned long long stratum_groupCacheBytes(int entries);

@@ -454,6 +454,15 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
       r1 = cacheRecord(cache, e, min(lane + 32, kEntryRecords - 1));
       const bool same = lane < 9 ? tag == row : lane != 9 || tag == uint32_t(g);
       if (__all_sync(0xffffffffu, same)) return int(__shfl_sync(0xffffffffu, tag, 10));
+    } else {
+      const int f = filledNow(cache, word, slot, g);
+      if (f >= 0) {
+        const uint32_t tag = lane < kEntryTagWords ? __ldcg(entryTag(cache, uint32_t(f)) + lane) : 0u;
+        r0 = freshRecord(cache, f, lane);
+        r1 = freshRecord(cache, f, min(lane + 32, kEntryRecords - 1));
+        const bool same = lane < 9 ? tag == row : lane != 9 || tag == uint32_t(g);
+        if (__all_sync(0xffffffffu, same)) return int(__shfl_sync(0xffffffffu, tag, 10));
+      }
     }
   }
   if (held < 0) {
