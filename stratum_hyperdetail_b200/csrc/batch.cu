@@ -98,8 +98,9 @@ __global__ void cacheInitK(uint32_t* base, uint32_t entries) {
 // `bandTiles`: band tiles to give out over all views: twice the warps the device
 // holds.  Warm trace of one 640x360 view, street / rooftop / aerial / canal / avenue:
 // no band 417 / 486 / 637 / 399 / 460 us, once the warps 363 / 484 / 629 / 359 / 285,
-// twice 309 / 355 / 634 / 248 / 291, four times 324 / 377 / 723 / 262 / 310.  A view
-// of a large batch still gets one tile row.
+// twice 309 / 355 / 634 / 248 / 291, four times 324 / 377 / 723 / 262 / 310.  Views
+// of a large batch get none: there the other views' tiles fill the device (one tile row
+// each made twelve mixed views 0.5 % slower).
 __global__ void prologueK(stratum_view* V, int n, int order, int bandTiles, BatchScratch* S) {
   for (int v = int(threadIdx.x); v < n; v += int(blockDim.x)) {
     S->view[v].frame = makeFrame(V[v].C, V[v].Origin);
@@ -108,9 +109,9 @@ __global__ void prologueK(stratum_view* V, int n, int order, int bandTiles, Batc
     Band& b = S->view[v].band;
     b.horizon = b.row0 = b.row1 = 0;
     if (W > 0 && H > 0) {
-      const int rows = (H + kTileH - 1) / kTileH, want = max(1, bandTiles / n / (V[v].tilesX * kTileH)), band = min(want, rows);
+      const int rows = (H + kTileH - 1) / kTileH, want = bandTiles / n / (V[v].tilesX * kTileH), band = min(want, rows);
       b.horizon = horizonRow(S->view[v].frame.cam, H);
-      b.row0 = min(max(b.horizon / kTileH - band / 2, 0), rows - band);
+      b.row0 = min(max(b.horizon / kTileH - band / 2, 0), rows - band);  // may be none
       b.row1 = b.row0 + band;
     }
     if (V[v].Groups) {  // this launch's epoch; a full cache starts again now and then
