@@ -143,7 +143,8 @@ struct CoopRay {
   float cone, best;
   int fid, wslot, wcx, wcz;  // winner: group*64+index, slot and DDA cell of its lot
   // lot DDA
-  float t, tx, tz, dx, dz, farT;
+  float t, tx, tz, farT;
+  f3 inv;  // inverse of rd
   int cx, cz, sx, sz, ddaSteps;
   // current lot
   int slot, lcx, lcz;
@@ -182,11 +183,16 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.cz = int(floorf((start.z + 18.0f) / kCell));
   r.sx = rd.x > 0.0f ? 1 : -1;
   r.sz = rd.z > 0.0f ? 1 : -1;
-  float ix = guardedInv(rd.x), iz = guardedInv(rd.z);
-  r.tx = (float(r.cx) * kCell + (r.sx > 0 ? 18.0f : -18.0f) - ro.x) * ix;
-  r.tz = (float(r.cz) * kCell + (r.sz > 0 ? 18.0f : -18.0f) - ro.z) * iz;
-  r.dx = kCell * fabsf(ix);
-  r.dz = kCell * fabsf(iz);
+  r.inv = invDir(rd);
+  r.tx = (float(r.cx) * kCell + (r.sx > 0 ? 18.0f : -18.0f) - ro.x) * r.inv.x;
+  r.tz = (float(r.cz) * kCell + (r.sz > 0 ? 18.0f : -18.0f) - ro.z) * r.inv.z;
+}
+// invDir(toLot(d, turn)) from invDir(d): the same permutation with the same signs,
+// except for an exactly zero component, whose guarded inverse is positive either way.
+SD f3 invToLot(f3 inv, f3 d, int turn) {
+  const f3 p = toLot(inv, turn);
+  return mk(d.x == 0.0f && (turn == 2) ? inv.x : (d.z == 0.0f && turn == 3 ? inv.z : p.x), p.y,
+            d.z == 0.0f && turn == 2 ? inv.z : (d.x == 0.0f && turn == 1 ? inv.x : p.z));
 }
 
 // Inner node where the paths to two leaves part.
@@ -251,10 +257,11 @@ SD void coopEnterLot(CoopRay& r, const float* __restrict__ W, const float4* __re
     f3 cp = mk(float(r.cx) * kCell + c.z, 0.0f, float(r.cz) * kCell + c.w);
     r.lr = toLot(r.ro - cp, turn);
     r.ld = toLot(r.rd, turn);
-    r.inv0 = invDir(r.ld);
+    r.inv0 = invToLot(r.inv, r.rd, turn);
     // the DDA steps to the next cell now; the reference does it after the
     // lot's query, and the next test reads only t and the (later) best
-    if (r.tx < r.tz) { r.t = r.tx; r.tx += r.dx; r.cx += r.sx; } else { r.t = r.tz; r.tz += r.dz; r.cz += r.sz; }
+    if (r.tx < r.tz) { r.t = r.tx; r.tx += kCell * fabsf(r.inv.x); r.cx += r.sx; }
+    else { r.t = r.tz; r.tz += kCell * fabsf(r.inv.z); r.cz += r.sz; }
     if (nodeEntry(N, r.slot * kNodes + 1, r.lr, r.inv0, r.best) < r.best) r.state = kLotPending;
   }
 }
