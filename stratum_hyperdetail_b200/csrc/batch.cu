@@ -268,10 +268,14 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
   retire(&S->counters[kTraceNext], &S->counters[kTraceDone], THREADS);
 }
 
-// STRATUM_SHADE_OCC / THREADS resident blocks: 1536 threads per SM (40 registers,
-// some spills) measured fastest; shading is latency-bound.
+// STRATUM_SHADE_OCC / THREADS resident blocks of the material pass: 1280 threads
+// per SM (six 1600x900 views 392 us; 1024 397, 1536 404); STRATUM_LIGHT_OCC of
+// the lighting pass: 1536 (40 registers, some spills: 736 us; 1024 764).
 #ifndef STRATUM_SHADE_OCC
-#define STRATUM_SHADE_OCC 1536
+#define STRATUM_SHADE_OCC 1280
+#endif
+#ifndef STRATUM_LIGHT_OCC
+#define STRATUM_LIGHT_OCC 1536
 #endif
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, STRATUM_SHADE_OCC / THREADS) shadeViewsK(const stratum_view* __restrict__ V, int n, int grab, int order,
@@ -311,13 +315,14 @@ __global__ void __launch_bounds__(THREADS, STRATUM_SHADE_OCC / THREADS) shadeVie
   retire(&S->counters[kShadeNext], &S->counters[kShadeDone], THREADS);
 }
 
-// STRATUM_RESOLVE_OCC / THREADS resident blocks (0: the compiler's choice;
-// 1024, 1536 and 2048 threads per SM measured the same).
+// STRATUM_RESOLVE_OCC / THREADS resident blocks: the taps' loads are what it waits
+// for (1024 threads per SM 611 us for the six views; 1280 630, 1536 648, the
+// compiler's choice of 72 registers 639).
 #ifndef STRATUM_RESOLVE_OCC
-#define STRATUM_RESOLVE_OCC 0
+#define STRATUM_RESOLVE_OCC 1024
 #endif
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, STRATUM_SHADE_OCC / THREADS) lightViewsK(const stratum_view* __restrict__ V,
+__global__ void __launch_bounds__(THREADS, STRATUM_LIGHT_OCC / THREADS) lightViewsK(const stratum_view* __restrict__ V,
                                                                                 int n, int grab, int order,
                                                                                 BatchScratch* S) {
   const int lane = int(threadIdx.x & 31);

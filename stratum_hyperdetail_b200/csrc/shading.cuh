@@ -12,6 +12,13 @@ namespace st {
 // height field and powf for all shading call sites: inlined at every use they
 // multiply the kernel's code and it stalls on instruction fetch.  Same
 // arithmetic, same bits.
+//
+// What bounds shading is instruction issue, then instruction fetch.  Work whose
+// result is certain is left out below, always to the same bits: noise with a
+// weight of exactly 0, the sun's powers where they are 0, a lot's inverse
+// directions by permuting the light's, masses below the point, and resolve taps
+// that cannot occlude.  Six 1600x900 views: material 455 -> 392 us, light 875 -> 736,
+// resolve 712 -> 611.
 static __device__ __noinline__ float noise2D(float x, float y) { return noise2(x, y); }
 static __device__ __noinline__ float fbm2D(float x, float y) { return fbm2(x, y); }
 static __device__ __noinline__ float masonryHeightD(float u, float v, int material) { return masonryHeight(u, v, material); }
@@ -29,7 +36,9 @@ static __device__ __noinline__ f3 skyColor(f3 rd, f3 sun) {
   float elev = sat(rd.y);
   f3 c = mix(mk(0.62f, 0.69f, 0.72f), mk(0.13f, 0.30f, 0.52f), powD(elev, 0.45f));
   float sd = fmaxf(0.0f, dot(rd, sun));
-  c = c + mk(1.1f, 0.62f, 0.22f) * powD(sd, 18.0f) + mk(9.0f, 6.0f, 3.2f) * powD(sd, 2600.0f);
+  // (0^18 is 0, and 0.95^2600 = 2^-192 is 0 in a float)
+  if (sd > 0.0f) c = c + mk(1.1f, 0.62f, 0.22f) * powD(sd, 18.0f);
+  if (sd > 0.95f) c = c + mk(9.0f, 6.0f, 3.2f) * powD(sd, 2600.0f);
   if (rd.y > 0.025f) {
     float cloud = fbm2D(rd.x / (rd.y + 0.20f) * 1.8f + 16.0f, rd.z / (rd.y + 0.20f) * 1.8f);
     float veil = smooth(0.46f, 0.70f, cloud) * smooth(0.02f, 0.2f, rd.y) * 0.55f;
@@ -53,11 +62,14 @@ SD f3 mineralCell(float u, float v, int seed) {
   return mk(sqrtf(nearest), value, sqrtf(second) - sqrtf(nearest));
 }
 SD float microRelief(float u, float v, float fp) {
+  const float mid = freqWeight(fp, 277.0f), high = freqWeight(fp, 911.0f);
   float value = (noise2D(u * 83.0f, v * 83.0f) - 0.5f) * 0.0016f * freqWeight(fp, 83.0f);
-  value += (noise2D(u * 277.0f + 8.7f, v * 277.0f) - 0.5f) * 0.00048f * freqWeight(fp, 277.0f);
-  value += (noise2D(u * 911.0f, v * 911.0f - 13.9f) - 0.5f) * 0.00013f * freqWeight(fp, 911.0f);
+  if (mid > 0.0f) value += (noise2D(u * 277.0f + 8.7f, v * 277.0f) - 0.5f) * 0.00048f * mid;
+  if (high > 0.0f) value += (noise2D(u * 911.0f, v * 911.0f - 13.9f) - 0.5f) * 0.00013f * high;
   return value;
 }
+// Terms whose frequency weight is exactly 0 at this footprint (1.1 / frequency and
+// beyond) leave the colour as it is, so their noise is not evaluated.
 static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, float fp, f3 foundation) {
   float u, v;
   masonryUV(p, n, u, v);
@@ -87,16 +99,20 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
       float powder = (noise2D(u * 740.0f, v * 740.0f) - 0.5f) * freqWeight(fp, 740.0f);
       c = c * (1.0f + powder * (joint > 0.5f ? 0.50f : 0.24f));
     }
-    float crack = fabsf(sinf(u * 8.4f + fbm2D(u * 2.4f, v * 2.4f) * 5.0f + v * 1.3f));
-    float fracture = (1.0f - smooth(0.012f, 0.042f + fp * 4.0f, crack)) * smooth(0.48f, 0.72f, noise2D(u * 1.4f, v * 1.4f));
-    c = c * (1.0f - fracture * 0.45f * freqWeight(fp, 15.0f));
+    const float cracks = freqWeight(fp, 15.0f);
+    if (cracks > 0.0f) {
+      float crack = fabsf(sinf(u * 8.4f + fbm2D(u * 2.4f, v * 2.4f) * 5.0f + v * 1.3f));
+      float fracture = (1.0f - smooth(0.012f, 0.042f + fp * 4.0f, crack)) * smooth(0.48f, 0.72f, noise2D(u * 1.4f, v * 1.4f));
+      c = c * (1.0f - fracture * 0.45f * cracks);
+    }
     float moss = (1.0f - smooth(0.1f, 3.1f, p.y)) * smooth(0.44f, 0.69f, noise2D(u * 1.3f, v * 0.3f));
     c = mix(c, mk(0.095f, 0.125f, 0.046f), moss * 0.7f);
   } else if (mat == 2 || mat == 14) {  // slate / terracotta tiles
     c = mat == 2 ? mk(0.14f, 0.19f, 0.22f) : mk(0.38f, 0.125f, 0.048f);
     float tile = fract(u * 3.7f), row = fract(v * 4.4f);
     float seam = (1.0f - smooth(0.01f, 0.07f, tile)) + (1.0f - smooth(0.02f, 0.11f, row));
-    c = c * (0.78f + 0.26f * lerp(0.5f, noise2D(u * 7.2f, v * 7.2f), freqWeight(fp, 7.2f)) -
+    const float mottle = freqWeight(fp, 7.2f);
+    c = c * (0.78f + 0.26f * (mottle > 0.0f ? lerp(0.5f, noise2D(u * 7.2f, v * 7.2f), mottle) : 0.5f) -
              sat(seam) * 0.25f * freqWeight(fp, 4.4f));
   } else if (mat == 3) {  // copper patina
     float patina = smooth(0.28f, 0.64f, fbm2D(u * 2.1f, v * 2.1f));
@@ -105,8 +121,8 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
     c = c * (1.0f - seam * 0.4f * freqWeight(fp, 1.8f));
   } else if (mat == 4) c = mk(0.045f, 0.084f, 0.093f);
   else if (mat == 5) {
-    float grain = sinf(u * 49.0f + fbm2D(u * 2.0f, v * 0.5f) * 8.0f);
-    c = mk(0.12f, 0.07f, 0.039f) * (1.0f + grain * 0.12f * fine);
+    c = mk(0.12f, 0.07f, 0.039f);
+    if (fine > 0.0f) c = c * (1.0f + sinf(u * 49.0f + fbm2D(u * 2.0f, v * 0.5f) * 8.0f) * 0.12f * fine);
   } else if (mat == 6) c = mk(0.075f, 0.091f, 0.087f) * (0.8f + noise2D(u * 30.0f, v * 30.0f) * 0.3f);
   else if (mat == 7) {
     float leaves = fbm2D(p.x * 8.0f + p.y * 6.0f, p.z * 8.0f);
@@ -114,7 +130,8 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
   } else if (mat == 8) c = mk(0.70f, 0.43f, 0.13f);
   else if (mat == 9) c = mk(0.035f, 0.115f, 0.12f);
   else if (mat == 10) {
-    float grit = lerp(0.5f, fbm2D(u * 45.0f, v * 45.0f), freqWeight(fp, 45.0f));
+    const float gravel = freqWeight(fp, 45.0f);
+    float grit = gravel > 0.0f ? lerp(0.5f, fbm2D(u * 45.0f, v * 45.0f), gravel) : 0.5f;
     c = mk(0.16f, 0.17f, 0.16f) * (0.72f + grit * 0.4f);
   } else if (mat == 11) {
     int row = int(floorf(v / 0.45f));
@@ -147,10 +164,10 @@ static __device__ __noinline__ float buildingShadow(const float* __restrict__ W,
   f3 ro = p + light * 0.08f;
   int cx = int(floorf((ro.x + 18.0f) / kCell)), cz = int(floorf((ro.z + 18.0f) / kCell));
   int sx = light.x > 0.0f ? 1 : -1, sz = light.z > 0.0f ? 1 : -1;
-  float ix = guardedInv(light.x), iz = guardedInv(light.z);
-  float tx = (float(cx) * kCell + (sx > 0 ? 18.0f : -18.0f) - ro.x) * ix;
-  float tz = (float(cz) * kCell + (sz > 0 ? 18.0f : -18.0f) - ro.z) * iz;
-  float dx = kCell * fabsf(ix), dz = kCell * fabsf(iz), t = 0.0f;
+  const f3 inv = invDir(light);
+  float tx = (float(cx) * kCell + (sx > 0 ? 18.0f : -18.0f) - ro.x) * inv.x;
+  float tz = (float(cz) * kCell + (sz > 0 ? 18.0f : -18.0f) - ro.z) * inv.z;
+  float dx = kCell * fabsf(inv.x), dz = kCell * fabsf(inv.z), t = 0.0f;
 #pragma unroll 1
   for (int step = 0; step < 64; step++) {
     if (t > limit) break;
@@ -158,8 +175,8 @@ static __device__ __noinline__ float buildingShadow(const float* __restrict__ W,
                                                               : describe(shiftAddr(o0, o1, o2, o3, cx, cz), worldSeed);
     if (l.type < 3) {
       f3 cp = mk(float(cx) * kCell + l.ox, 0.0f, float(cz) * kCell + l.oz);
-      f3 lr = toLot(ro - cp, l.turn), ld = toLot(light, l.turn);
-      Span s = slab(lr, ld, mk(-l.w + 0.05f, 4.1f, -l.d + 0.05f), mk(l.w - 0.05f, l.h, l.d - 0.05f));
+      f3 lr = toLot(ro - cp, l.turn);
+      Span s = slabInv(lr, invToLot(inv, light, l.turn), mk(-l.w + 0.05f, 4.1f, -l.d + 0.05f), mk(l.w - 0.05f, l.h, l.d - 0.05f));
       if (s.hi > fmaxf(0.06f, s.lo) && s.lo < limit) return 0.06f;
     }
     if (tx < tz) { t = tx; tx += dx; cx += sx; } else { t = tz; tz += dz; cz += sz; }
@@ -174,7 +191,7 @@ SD float ambientVisibility(const float* __restrict__ W, uint32_t o0, uint32_t o2
 #pragma unroll 1
     for (int x = -1; x <= 1; x++) {
       LotDesc l = loadLot(W, tableSlot(o0, o2, cx + x, cz + z));
-      if (l.type >= 3) continue;
+      if (l.type >= 3 || l.h <= p.y) continue;  // (a mass below the point occludes nothing)
       f3 q = toLot(p - mk(float(cx + x) * kCell + l.ox, 0.0f, float(cz + z) * kCell + l.oz), l.turn);
       float xx = fmaxf(0.0f, fabsf(q.x) - l.w), zz = fmaxf(0.0f, fabsf(q.z) - l.d);
       float dist = sqrtf(xx * xx + zz * zz);
@@ -278,16 +295,18 @@ SD f3 pixelLight(const float* __restrict__ W, const FrameConst& F, const Surface
   f3 n = s.n, result;
   f3 originalN = n;
   if ((mat == 0 || mat == 1) && fabsf(qn.y) < 0.5f) {  // mortar relief normal by central differences
-    float eps = fmaxf(0.002f, sfp * 0.6f);
-    float du = (masonryHeightD(u + eps, v, mat) - masonryHeightD(u - eps, v, mat)) / (2.0f * eps);
-    float dv = (masonryHeightD(u, v + eps, mat) - masonryHeightD(u, v - eps, mat)) / (2.0f * eps);
-    if (sfp < 0.005f) {
-      float me = fmaxf(0.00016f, sfp * 0.8f);
-      du += (microRelief(u + me, v, sfp) - microRelief(u - me, v, sfp)) / (2.0f * me);
-      dv += (microRelief(u, v + me, sfp) - microRelief(u, v - me, sfp)) / (2.0f * me);
+    const float fade = freqWeight(sfp, 5.0f);
+    float eps = fmaxf(0.002f, sfp * 0.6f), du = 0.0f, dv = 0.0f;
+    if (fade > 0.0f) {
+      du = (masonryHeightD(u + eps, v, mat) - masonryHeightD(u - eps, v, mat)) / (2.0f * eps);
+      dv = (masonryHeightD(u, v + eps, mat) - masonryHeightD(u, v - eps, mat)) / (2.0f * eps);
+      if (sfp < 0.005f) {
+        float me = fmaxf(0.00016f, sfp * 0.8f);
+        du += (microRelief(u + me, v, sfp) - microRelief(u - me, v, sfp)) / (2.0f * me);
+        dv += (microRelief(u, v + me, sfp) - microRelief(u, v - me, sfp)) / (2.0f * me);
+      }
     }
     f3 tangent = fabsf(qn.x) > 0.5f ? mk(0.0f, 0.0f, 1.0f) : mk(1.0f, 0.0f, 0.0f);
-    float fade = freqWeight(sfp, 5.0f);
     f3 localN = unit(qn - tangent * (du * fade) - mk(0.0f, dv * fade, 0.0f));
     n = fromLot(localN, s.lot.turn);
   }
@@ -372,13 +391,35 @@ SD void resolvePixel(f3 c, float4* Hist, uint32_t* Px, const FrameConst& F, cons
     float4 s4 = Surf[b];
     f3 n = mk(s4.x, s4.y, s4.z);
     float occ = 0.0f;
+    const float rowInv = 1.08f / float(height), bound = 2e-6f * (fabsf(ro.x) + fabsf(ro.y) + fabsf(ro.z) + 2.0f * h4.x + 2.0f);
+    const float reach = 2.0f + 2.0f * bound, slack = bound * (0.5f + 4.0f * (fabsf(n.x) + fabsf(n.y) + fabsf(n.z)));
+    const f3 mine = point - ro;
     float radius = clampv(float(height) / (fmaxf(h4.x, 0.5f) * 1.08f) * 0.8f, 3.0f, 28.0f);
+    // a tap's distance and id are loaded while the one before it is evaluated
+    const float2* hit2 = reinterpret_cast<const float2*>(Hit);
+    auto tapX = [&](int k) { return int(clampv(float(x) + taps.c[k] * radius, 0.0f, float(width - 1))); };
+    auto tapY = [&](int k) { return int(clampv(float(y) + taps.s[k] * radius, 0.0f, float(height - 1))); };
+    int nx = tapX(0), ny = tapY(0);
+    float2 next = hit2[2 * (size_t(ny) * width + nx)];
 #pragma unroll 1
     for (int k = 0; k < 8; k++) {
-      int xx = int(clampv(float(x) + taps.c[k] * radius, 0.0f, float(width - 1)));
-      int yy = int(clampv(float(y) + taps.s[k] * radius, 0.0f, float(height - 1)));
-      float4 o4 = Hit[size_t(yy) * width + xx];
+      const int xx = nx, yy = ny;
+      const float2 o4 = next;
+      if (k < 7) {
+        nx = tapX(k + 1);
+        ny = tapY(k + 1);
+        next = hit2[2 * (size_t(ny) * width + nx)];
+      }
       if (int(o4.y) != kSkyId) {
+        // Most taps lie on the same flat surface or too far behind and add exactly
+        // 0; a quick estimate of the tap's offset, good to `bound` (the rounding of
+        // both computations), tells so without the exact square roots and divisions.
+        const float sx = (float(xx) + 0.5f + F.cam.jx - 0.5f * float(width)) * rowInv;
+        const float sy = (0.5f * float(height) - float(yy) - 0.5f - F.cam.jy) * rowInv;
+        const f3 far = F.cam.fwd + F.cam.right * sx + F.cam.up * sy;
+        const f3 d = far * (rsqrtf(dot(far, far)) * o4.x) - mine;
+        const float dd = dot(d, d), most = dot(n, d) + slack;
+        if (dd > reach * reach || most <= 0.0f || most * most < 0.0142f * dd) continue;
         f3 other = ro + primaryDir(F.cam, xx, yy, width, height) * o4.x, delta = other - point;
         float l = len(delta);
         if (l > 0.04f && l < 2.0f) occ += fmaxf(0.0f, dot(n, delta / l) - 0.12f) * expf(-l * 1.4f) * 0.28f;

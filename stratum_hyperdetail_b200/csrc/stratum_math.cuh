@@ -265,6 +265,13 @@ HD f3 toLot(f3 p, int turn) {
 }
 HD f3 fromLot(f3 p, int turn) { return toLot(p, (4 - turn) % 4); }
 
+// invDir(toLot(d, turn)) from invDir(d): the same permutation with the same signs,
+// except for an exactly zero component, whose guarded inverse is positive either way.
+SD f3 invToLot(f3 inv, f3 d, int turn) {
+  const f3 p = toLot(inv, turn);
+  return mk(d.x == 0.0f && (turn == 2) ? inv.x : (d.z == 0.0f && turn == 3 ? inv.z : p.x), p.y,
+            d.z == 0.0f && turn == 2 ? inv.z : (d.x == 0.0f && turn == 1 ? inv.x : p.z));
+}
 // Least and greatest value over a full warp (every lane calls).
 SD float warpMin(float v) {
   float r;

@@ -187,13 +187,6 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.tx = (float(r.cx) * kCell + (r.sx > 0 ? 18.0f : -18.0f) - ro.x) * r.inv.x;
   r.tz = (float(r.cz) * kCell + (r.sz > 0 ? 18.0f : -18.0f) - ro.z) * r.inv.z;
 }
-// invDir(toLot(d, turn)) from invDir(d): the same permutation with the same signs,
-// except for an exactly zero component, whose guarded inverse is positive either way.
-SD f3 invToLot(f3 inv, f3 d, int turn) {
-  const f3 p = toLot(inv, turn);
-  return mk(d.x == 0.0f && (turn == 2) ? inv.x : (d.z == 0.0f && turn == 3 ? inv.z : p.x), p.y,
-            d.z == 0.0f && turn == 2 ? inv.z : (d.x == 0.0f && turn == 1 ? inv.x : p.z));
-}
 
 // Inner node where the paths to two leaves part.
 SD int forkOf(int a, int b) { return (kGroups + a) >> (32 - __clz(a ^ b)); }
