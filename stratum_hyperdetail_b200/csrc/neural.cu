@@ -7,6 +7,7 @@
 // the samples' work rows and the gradient stay in shared memory and the phases
 // are separated by block barriers.
 #include "common_api.cuh"
+#include "frame_init.cuh"
 #include "neural.cuh"
 
 namespace st {
@@ -28,7 +29,10 @@ __global__ void initNeuralK(float* W, float* M, float* V, float* Brain, int seed
 
 constexpr int kStepThreads = 320;  // >= 291 parameters and >= 64 samples
 
-// One training step (learning.cu:11-58) on a frame's Hit/Surface.
+// One training step (learning.cu:11-58) on a frame's Hit/Surface.  One block, so
+// what bounds it is the longest chain of dependent steps, not work: every phase is
+// spread over all threads as far as its sums allow (their order is kept).  With
+// a thread a sample, and then a thread a parameter, it took 30 us; now STEP_US.
 __global__ void __launch_bounds__(kStepThreads) materialStepK(const float* __restrict__ World,
                                                              const uint32_t* __restrict__ O,
                                                              const float* __restrict__ C,
@@ -36,59 +40,86 @@ __global__ void __launch_bounds__(kStepThreads) materialStepK(const float* __res
                                                              const float* __restrict__ Surface, float* W, float* M,
                                                              float* V, float* Brain, float* WorkOut, int width,
                                                              int height) {
+  constexpr int kTrials = 6;
   __shared__ float work[kNnBatch * kNnWs];
-  __shared__ float grad[kNnParams];
+  __shared__ float weight[kNnParams], grad[kNnParams], delta[kNnTrain * kNnHidden], decay[2];
+  __shared__ float su[kNnBatch], sv[kNnBatch], seedOf[kNnBatch];
+  __shared__ int pick[kNnBatch];
   __shared__ FrameConst F;
   if (!materialTrainNow(C)) return;  // uniform over the block
   const int i = int(threadIdx.x);
-  if (i == 0) F = makeFrame(C, O);
-  __syncthreads();
+  for (int k = i; k < kNnBatch * kNnWs; k += kStepThreads) work[k] = 0.0f;
+  if (i < kNnBatch) pick[i] = -1;
+  if (i < kNnParams) weight[i] = W[i];
+  frameInit(F, C, O);
   // prepare (learning.cu:11-24): the last of six hashed pixels that hit brick or stone
-  if (i < kNnBatch) {
-    float* w = work + i * kNnWs;
-    int chosen = -1;
-    for (int trial = 0; trial < 6; trial++) {
-      const int px = int(hash1(i * 1877 + trial * 331 + int(C[6]) * 59) * float(width * height));
-      const int id = int(Hit[px * 4 + 1]);
-      if (id >= 0) {
-        const int mat = int(Hit[px * 4 + 2]);
-        if (mat == 0 || mat == 1) chosen = px;
-      }
-    }
-    for (int j = 0; j < kNnWs; j++) w[j] = 0.0f;
-    if (chosen >= 0) {
-      const int x = chosen % width, y = chosen / width;
-      const f3 rd = primaryDir(F.cam, x, y, width, height);
-      const float4 h = reinterpret_cast<const float4*>(Hit)[chosen];
-      const float4 s = reinterpret_cast<const float4*>(Surface)[chosen];
-      SurfacePoint sp;
-      surfacePoint(World, F, h, s, rd, height, sp);
+  auto pixelOf = [&](int sample, int trial) {
+    return int(hash1(sample * 1877 + trial * 331 + int(C[6]) * 59) * float(width * height));
+  };
+  for (int k = i; k < kNnBatch * kTrials; k += kStepThreads) {
+    const int sample = k / kTrials, trial = k % kTrials;
+    const float4 h = reinterpret_cast<const float4*>(Hit)[pixelOf(sample, trial)];
+    if (int(h.y) >= 0) {
       const int mat = int(h.z);
-      for (int j = 0; j < kNnInputs; j++) w[j] = nnFeature(j, sp.u, sp.v, h.w, mat);
-      const f3 target = substrate(sp.u, sp.v, h.w, mat);
+      if (mat == 0 || mat == 1) atomicMax(&pick[sample], trial);
+    }
+  }
+  __syncthreads();
+  if (i < kNnBatch && pick[i] >= 0) {
+    float* w = work + i * kNnWs;
+    const int chosen = pixelOf(i, pick[i]), x = chosen % width, y = chosen / width;
+    const f3 rd = primaryDir(F.cam, x, y, width, height);
+    const float4 h = reinterpret_cast<const float4*>(Hit)[chosen];
+    const float4 s = reinterpret_cast<const float4*>(Surface)[chosen];
+    SurfacePoint sp;
+    surfacePoint(World, F, h, s, rd, height, sp);
+    su[i] = sp.u; sv[i] = sp.v; seedOf[i] = h.w;
+    w[kNnValid] = 1.0f;
+    w[kNnMat] = float(int(h.z));
+  }
+  __syncthreads();
+  for (int k = i; k < kNnBatch * (kNnInputs + 1); k += kStepThreads) {  // target and inputs, a kind to a run of threads
+    const int j = k / kNnBatch, sample = k % kNnBatch;
+    float* w = work + sample * kNnWs;
+    if (pick[sample] < 0) continue;
+    const int mat = int(w[kNnMat]);
+    if (j == 0) {
+      const f3 target = substrate(su[sample], sv[sample], seedOf[sample], mat);
       w[kNnTarget] = target.x; w[kNnTarget + 1] = target.y; w[kNnTarget + 2] = target.z;
-      w[kNnValid] = 1.0f;
-      w[kNnMat] = float(mat);
+    } else {
+      w[j - 1] = nnFeature(j - 1, su[sample], sv[sample], seedOf[sample], mat);
     }
   }
   __syncthreads();
   // forward (learning.cu:25-29)
-  if (i < kNnBatch) {
-    float* w = work + i * kNnWs;
-    for (int h = 0; h < kNnHidden; h++) {
-      float z = W[kNnB1 + h];
-      for (int j = 0; j < kNnInputs; j++) z += W[h * 8 + j] * w[j];
-      w[kNnHid + h] = nnActivate(z);
-    }
-    for (int o = 0; o < 3; o++) {
-      float z = W[kNnB2 + o];
-      for (int h = 0; h < kNnHidden; h++) z += W[kNnW2 + o * 24 + h] * w[kNnHid + h];
-      w[kNnOut + o] = z;
-    }
+  for (int k = i; k < kNnBatch * kNnHidden; k += kStepThreads) {
+    const int h = k / kNnBatch;
+    float* w = work + (k % kNnBatch) * kNnWs;
+    float z = weight[kNnB1 + h];
+    for (int j = 0; j < kNnInputs; j++) z += weight[h * 8 + j] * w[j];
+    w[kNnHid + h] = nnActivate(z);
   }
   __syncthreads();
+  for (int k = i; k < kNnBatch * 3; k += kStepThreads) {
+    const int o = k / kNnBatch;
+    float* w = work + (k % kNnBatch) * kNnWs;
+    float z = weight[kNnB2 + o];
+    for (int h = 0; h < kNnHidden; h++) z += weight[kNnW2 + o * 24 + h] * w[kNnHid + h];
+    w[kNnOut + o] = z;
+  }
+  __syncthreads();
+  // a hidden unit's error on each training sample (learning.cu:42-52)
+  for (int k = i; k < kNnTrain * kNnHidden; k += kStepThreads) {
+    const int h = k / kNnTrain, sample = k % kNnTrain;
+    const float* w = work + sample * kNnWs;
+    float d = 0.0f;
+    for (int o = 0; o < 3; o++) d += (w[kNnOut + o] - w[kNnTarget + o]) * weight[kNnW2 + o * 24 + h];
+    const float a = w[kNnHid + h];
+    d *= 1.0f - a * a;
+    delta[h * kNnTrain + sample] = d;
+  }
   // score on the 8 held-out samples and the validation gate (learning.cu:30-41)
-  if (i == 0) {
+  if (i == kStepThreads - 1) {
     float err = 0.0f, baseline = 0.0f, n = 0.0f;
     for (int k = kNnTrain; k < kNnBatch; k++) {
       const float* w = work + k * kNnWs;
@@ -112,44 +143,39 @@ __global__ void __launch_bounds__(kStepThreads) materialStepK(const float* __res
     }
     Brain[4] = Brain[1] >= 256.0f && Brain[2] < Brain[3] * 0.90f && Brain[2] < 0.0012f ? 1.0f : 0.0f;
   }
+  __syncthreads();
   // gradient over the 56 training samples (learning.cu:42-52)
+  float count = 0.0f;
+  for (int k = 0; k < kNnTrain; k++) count += work[k * kNnWs + kNnValid] > 0.5f ? 1.0f : 0.0f;
+  const float steps = Brain[0] + (count > 0.0f ? 1.0f : 0.0f);
   if (i < kNnParams) {
-    float g = 0.0f, count = 0.0f;
+    float g = 0.0f;
     for (int k = 0; k < kNnTrain; k++) {
       const float* w = work + k * kNnWs;
       if (w[kNnValid] > 0.5f) {
-        count += 1.0f;
-        if (i < kNnW2) {
-          const int h = i < kNnB1 ? i / 8 : i - kNnB1;
-          float d = 0.0f;
-          for (int o = 0; o < 3; o++) d += (w[kNnOut + o] - w[kNnTarget + o]) * W[kNnW2 + o * 24 + h];
-          const float a = w[kNnHid + h];
-          d *= 1.0f - a * a;
-          g += i < kNnB1 ? d * w[i % 8] : d;
-        } else if (i < kNnB2) {
-          const int o = (i - kNnW2) / 24, h = (i - kNnW2) % 24;
-          g += (w[kNnOut + o] - w[kNnTarget + o]) * w[kNnHid + h];
-        } else {
-          const int o = i - kNnB2;
-          g += w[kNnOut + o] - w[kNnTarget + o];
-        }
+        if (i < kNnB1) g += delta[(i / 8) * kNnTrain + k] * w[i % 8];
+        else if (i < kNnW2) g += delta[(i - kNnB1) * kNnTrain + k];
+        else if (i < kNnB2) g += (w[kNnOut + (i - kNnW2) / 24] - w[kNnTarget + (i - kNnW2) / 24]) * w[kNnHid + (i - kNnW2) % 24];
+        else g += w[kNnOut + i - kNnB2] - w[kNnTarget + i - kNnB2];
       }
     }
     grad[i] = clampv(g / fmaxf(1.0f, count), -0.8f, 0.8f);
-    if (i == 0) {
-      if (count > 0.0f) Brain[0] += 1.0f;
-      Brain[5] = count;
-    }
+  } else if (i == 296 || i == 297) {
+    decay[i - 296] = 1.0f - powR(i == 296 ? 0.9f : 0.999f, steps);
   }
   __syncthreads();
+  if (i == 0) {
+    Brain[0] = steps;
+    Brain[5] = count;
+  }
   // Adam (learning.cu:53-58)
-  if (i < kNnParams && Brain[5] >= 1.0f) {
+  if (i < kNnParams && count >= 1.0f) {
     const float g = grad[i];
     const float m = 0.9f * M[i] + 0.1f * g, v = 0.999f * V[i] + 0.001f * g * g;
     M[i] = m;
     V[i] = v;
-    const float mh = m / (1.0f - powR(0.9f, Brain[0])), vh = v / (1.0f - powR(0.999f, Brain[0]));
-    W[i] -= 0.002f * (mh / (sqrtf(vh) + 0.00001f) + 0.0001f * W[i]);
+    const float mh = m / decay[0], vh = v / decay[1];
+    W[i] = weight[i] - 0.002f * (mh / (sqrtf(vh) + 0.00001f) + 0.0001f * weight[i]);
   }
   if (WorkOut)
     for (int k = i; k < kNnBatch * kNnWs; k += kStepThreads) WorkOut[k] = work[k];
@@ -164,40 +190,46 @@ __global__ void predictSubstrateK(const float* __restrict__ W, const float* __re
   Out[size_t(i) * 3] = c.x; Out[size_t(i) * 3 + 1] = c.y; Out[size_t(i) * 3 + 2] = c.z;
 }
 
-// shadePixels with the surrogate in place of the procedural substrate of
-// brick and stone when C[16] enables it and the gate Brain[4] is open
-// (Stratum.cu:854); otherwise exactly the drop-in shadePixels.
-__global__ void __launch_bounds__(64) shadePixelsNeuralK(const float* __restrict__ World, const uint32_t* __restrict__ O,
-                                                        const float* __restrict__ C, const float* __restrict__ Hit,
-                                                        const float* __restrict__ Surface, float* Linear,
-                                                        const float* __restrict__ W, const float* __restrict__ Brain,
-                                                        int width, int height, int rowStart, int rowCount) {
+// The material half of shadePixels with the surrogate in place of the procedural
+// substrate of brick and stone when C[16] enables it and the gate Brain[4] is open
+// (Stratum.cu:854); otherwise exactly the drop-in's.  The lighting half follows as
+// its own kernel (shade.cu).
+constexpr int kNeuralThreads = 128;
+__global__ void __launch_bounds__(kNeuralThreads, 1024 / kNeuralThreads)
+    albedoNeuralK(const float* __restrict__ World, const uint32_t* __restrict__ O, const float* __restrict__ C,
+                  const float4* __restrict__ Hit, const float4* __restrict__ Surface, float4* Linear,
+                  const float* __restrict__ W, const float* __restrict__ Brain, int width, int height, int rowStart,
+                  int rowEnd) {
   __shared__ FrameConst F;
-  __shared__ int useNet;
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    F = makeFrame(C, O);
-    useNet = C[16] > 0.5f && Brain[4] > 0.5f;
+  frameInit(F, C, O);
+  const bool useNet = C[16] > 0.5f && Brain[4] > 0.5f;
+  const int tilesX = (width + 7) / 8, tiles = tilesX * ((rowEnd - rowStart + 3) / 4), warps = kNeuralThreads / 32;
+  const int lane = int(threadIdx.x & 31);
+#pragma unroll 1
+  for (int i = int(blockIdx.x) * warps + int(threadIdx.x >> 5); i < tiles; i += int(gridDim.x) * warps) {
+    const int x = (i % tilesX) * 8 + (lane & 7), y = rowStart + (i / tilesX) * 4 + (lane >> 3);
+    if (x >= width || y >= rowEnd) continue;
+    const size_t b = size_t(y) * width + x;
+    const f3 rd = primaryDir(F.cam, x, y, width, height);
+    const float4 h = Hit[b];
+    f3 c;
+    if (int(h.y) == kSkyId) {
+      c = skyColor(rd, F.sun);
+    } else {
+      SurfacePoint sp;
+      surfacePoint(World, F, h, Surface[b], rd, height, sp);
+      f3 base = substrateMean(sp.mat);
+      if (sp.mat == 0 || sp.mat == 1)
+        base = useNet ? predictSubstrate(W, sp.u, sp.v, sp.seed, sp.mat) : substrate(sp.u, sp.v, sp.seed, sp.mat);
+      c = surfaceColor(sp.q, sp.qn, sp.mat, sp.seed, sp.sfp, base) * paletteTint(sp.palette, sp.mat);
+    }
+    Linear[b] = make_float4(c.x, c.y, c.z, 1.0f);
   }
-  __syncthreads();
-  const int x = int(blockIdx.x * blockDim.x + threadIdx.x), y = rowStart + int(blockIdx.y * blockDim.y + threadIdx.y);
-  if (x >= width || y >= height || y >= rowStart + rowCount) return;
-  const size_t b = size_t(y) * width + x;
-  const f3 rd = primaryDir(F.cam, x, y, width, height);
-  const float4 h = reinterpret_cast<const float4*>(Hit)[b], s = reinterpret_cast<const float4*>(Surface)[b];
-  f3 c;
-  if (int(h.y) == kSkyId) {
-    c = skyColor(rd, F.sun);
-  } else {
-    SurfacePoint sp;
-    surfacePoint(World, F, h, s, rd, height, sp);
-    f3 base = substrateMean(sp.mat);
-    if (sp.mat == 0 || sp.mat == 1)
-      base = useNet ? predictSubstrate(W, sp.u, sp.v, sp.seed, sp.mat) : substrate(sp.u, sp.v, sp.seed, sp.mat);
-    const f3 albedo = surfaceColor(sp.q, sp.qn, sp.mat, sp.seed, sp.sfp, base) * paletteTint(sp.palette, sp.mat);
-    c = pixelLight(World, F, sp, rd, int(h.y), albedo);
-  }
-  reinterpret_cast<float4*>(Linear)[b] = make_float4(c.x, c.y, c.z, 1.0f);
 }
+
+// The lighting half of shadePixels (shade.cu).
+int lightRows(const float* World, const unsigned* Origin, const float* C, const float* Hit, const float* Surface,
+              float* Linear, int width, int height, int rowStart, int rows, cudaStream_t stream);
 
 }  // namespace st
 
@@ -236,10 +268,13 @@ int stratum_shadePixelsNeural(const float* World, const unsigned* Origin, const 
   if (rowStart < 0 || rowCount < 0) return STRATUM_EINVAL;
   const int rows = rowCount < height - rowStart ? rowCount : height - rowStart;
   if (rows <= 0) return STRATUM_OK;
-  dim3 grid((width + 7) / 8, (rows + 7) / 8);
-  shadePixelsNeuralK<<<grid, dim3(8, 8), 0, asStream(stream)>>>(World, Origin, C, Hit, Surface, Linear, W, Brain,
-                                                              width, height, rowStart, rowCount);
-  return launchStatus();
+  const int need = ((width + 7) / 8 * ((rows + 3) / 4) + 3) / 4, most = 148 * (1024 / kNeuralThreads);
+  albedoNeuralK<<<need < most ? need : most, kNeuralThreads, 0, asStream(stream)>>>(
+      World, Origin, C, reinterpret_cast<const float4*>(Hit), reinterpret_cast<const float4*>(Surface),
+      reinterpret_cast<float4*>(Linear), W, Brain, width, height, rowStart, rowStart + rows);
+  const int s = launchStatus();
+  return s != STRATUM_OK ? s
+                         : lightRows(World, Origin, C, Hit, Surface, Linear, width, height, rowStart, rows, asStream(stream));
 }
 
 }  // extern "C"

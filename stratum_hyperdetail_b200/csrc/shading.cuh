@@ -230,11 +230,10 @@ SD FrameConst makeFrame(const float* C, const uint32_t* O) {
   return f;
 }
 
-// Shading of one pixel (shade.cu:45-102) in three parts, so the batched path
-// can run the material and the lighting as two kernels (each a smaller body of
-// code for the instruction cache): the surface point, its albedo, its light.
-// shadePixel composes them; every path computes the same values in the same
-// order.
+// Shading of one pixel (shade.cu:45-102) in three parts, so that the material and
+// the lighting run as two kernels (each a smaller body of code for the
+// instruction cache): the surface point, its albedo, its light.  Every path
+// computes the same values in the same order.
 
 // A hit pixel's surface as shading sees it (shade.cu:45-70): the hit point in
 // the world and lot frames, the normal (flipped for foliage seen from inside),
@@ -357,15 +356,6 @@ SD f3 pixelLight(const float* __restrict__ W, const FrameConst& F, const Surface
   return result;
 }
 
-
-// Linear colour of one pixel (shade.cu:45-102).
-SD f3 shadePixel(const float* __restrict__ W, const FrameConst& F, float4 hit, float4 surf, f3 rd, int height) {
-  const int id = int(hit.y);
-  if (id == kSkyId) return skyColor(rd, F.sun);  // (a hit pixel's colour never reads the sky term)
-  SurfacePoint s;
-  surfacePoint(W, F, hit, surf, rd, height, s);
-  return pixelLight(W, F, s, rd, id, pixelAlbedo(s));
-}
 
 SD float aces(float x) { return sat(x * (2.51f * x + 0.03f) / (x * (2.43f * x + 0.59f) + 0.14f)); }
 
