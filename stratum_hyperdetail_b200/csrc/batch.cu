@@ -176,12 +176,12 @@ SD void retire(uint32_t* next, uint32_t* done, int threads) {
   }
 }
 
-// STRATUM_TRACE_OCC / THREADS resident blocks (rounded down).  512 threads per
-// SM (128 registers, a few bytes of spills): the six-view 1600x900 trace 4-5 %
-// faster than at 640 (96 registers, 88/136 bytes of spills), every pose faster;
-// 768 (80 registers, heavy spills) is slower still.
+// STRATUM_TRACE_OCC / THREADS resident blocks (rounded down).  576 threads per SM
+// (112 registers): six-view 1600x900 frame 5.95 ms, aerial trace 1.90; 448 threads
+// 6.07 / 1.96, 512 6.06 / 1.95, 640 5.98 / 1.91, 768 (80 registers, spills) 5.97 / 1.87
+// but the small views' slowest tiles 5-10 % slower.
 #ifndef STRATUM_TRACE_OCC
-#define STRATUM_TRACE_OCC 512
+#define STRATUM_TRACE_OCC 576
 #endif
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
       }
       const Camera cam = S->view[v].frame.cam;
       const uint32_t o0 = S->view[v].frame.o[0], o2 = S->view[v].frame.o[2];
-      f3 rd = primaryDir(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
+      f3 rd = primaryDir<Quotient>(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
       TraceResult r = traceWarp(V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2, cam.pos, rd,
                                 1.08f / float(H), inFrame, reinterpret_cast<WarpStage*>(stageBytes)[warp],
                                 groupCache(V[v].Groups));
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
     const bool inFrame = ok && x < W && y < H;
     const Camera cam = S->view[v].frame.cam;
     const uint32_t o0 = S->view[v].frame.o[0], o2 = S->view[v].frame.o[2];
-    const f3 rd = primaryDir(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
+    const f3 rd = primaryDir<Quotient>(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
     const TraceResult r = tracePooled<P>(sh, V, v, V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2,
                                          cam.pos, rd, 1.08f / float(H), inFrame);
     if (inFrame) storeTrace(V[v].Hit, V[v].Surface, size_t(y) * W + x, r);

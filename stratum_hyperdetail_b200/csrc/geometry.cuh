@@ -12,7 +12,7 @@ SD f3 intoFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(p.z, p.y, -p.x) 
 SD f3 outOfFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(-p.z, p.y, p.x) : p; }
 
 SD f3 leafNormal(int x, int y, int z, int seed) {  // geometry.cu:6-8
-  return unit(mk(hash2(x + y * 19, z, seed) - 0.5f, 0.25f + hash2(x - y, z + 91, seed) * 0.7f,
+  return Quotient::unit(mk(hash2(x + y * 19, z, seed) - 0.5f, 0.25f + hash2(x - y, z + 91, seed) * 0.7f,
                  hash2(z + y * 31, x, seed + 17) - 0.5f));
 }
 
@@ -21,9 +21,9 @@ static __device__ __noinline__ float foliageHit(f3 ro, f3 rd, f3 centre, f3 radi
   const float cell = 0.18f;
   float t = fmaxf(0.001f, begin) + 0.0001f;
   f3 pos = ro + rd * t;
-  int ix = int(floorf(pos.x / cell)), iy = int(floorf(pos.y / cell)), iz = int(floorf(pos.z / cell));
+  int ix = int(floorf(Quotient::div(pos.x, cell))), iy = int(floorf(Quotient::div(pos.y, cell))), iz = int(floorf(Quotient::div(pos.z, cell)));
   int sx = rd.x > 0.0f ? 1 : -1, sy = rd.y > 0.0f ? 1 : -1, sz = rd.z > 0.0f ? 1 : -1;
-  f3 inv = invDir(rd);
+  f3 inv = invDir<Quotient>(rd);
   float tx = (float(ix + (sx > 0 ? 1 : 0)) * cell - ro.x) * inv.x;
   float ty = (float(iy + (sy > 0 ? 1 : 0)) * cell - ro.y) * inv.y;
   float tz = (float(iz + (sz > 0 ? 1 : 0)) * cell - ro.z) * inv.z;
@@ -35,17 +35,17 @@ static __device__ __noinline__ float foliageHit(f3 ro, f3 rd, f3 centre, f3 radi
     float exitT = fminf(tx, fminf(ty, tz));
     f3 c = mk((float(ix) + 0.5f) * cell, (float(iy) + 0.5f) * cell, (float(iz) + 0.5f) * cell);
     f3 q = c - centre;
-    float ell = q.x * q.x / rx2 + q.y * q.y / ry2 + q.z * q.z / rz2;
+    float ell = Quotient::div(q.x * q.x, rx2) + Quotient::div(q.y * q.y, ry2) + Quotient::div(q.z * q.z, rz2);
     if (ell < 1.0f && hash2(ix + iy * 113, iz, seed) > 0.20f) {
       f3 n = leafNormal(ix, iy, iz, seed);
       float den = dot(rd, n);
       if (fabsf(den) > 0.00001f) {
-        float u = dot(c - ro, n) / den;
+        float u = Quotient::div(dot(c - ro, n), den);
         if (u >= t && u <= exitT) {
           f3 pp = ro + rd * u - c;
-          f3 tangent = unit(cross(n, mk(0.0f, 0.0f, 1.0f)));
+          f3 tangent = Quotient::unit(cross(n, mk(0.0f, 0.0f, 1.0f)));
           f3 bitangent = cross(n, tangent);
-          float a = dot(pp, tangent) / 0.125f, b = dot(pp, bitangent) / 0.062f;
+          float a = Quotient::div(dot(pp, tangent), 0.125f), b = Quotient::div(dot(pp, bitangent), 0.062f);
           if (a * a + b * b < 1.0f) return u;
         }
       }
@@ -65,7 +65,7 @@ static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f
   // is multiplied by exactly 0 and every step leaves t where it is; without this
   // return the four height-field steps of far walls took 13 % of the six-view
   // 1600x900 trace (6.80 -> 5.91 ms, aerial pose 2.89 -> 2.39 ms).
-  if (freqWeight(t * cone, 40.0f) == 0.0f) return t;
+  if (freqWeight<Quotient>(t * cone, 40.0f) == 0.0f) return t;
   f3 hp = p + d * t;
   float ex = fabsf(fabsf(hp.x) - h.x), ez = fabsf(fabsf(hp.z) - h.z);
   if (fabsf(fabsf(hp.y) - h.y) > 0.01f) {
@@ -79,8 +79,8 @@ static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f
         f3 wp = ro + rd * t;
         float u, v;
         masonryUV(wp, wn, u, v);
-        float disp = masonryHeight(u, v, f.material) * freqWeight(t * cone, 40.0f);
-        t = initial + disp / denom;
+        float disp = masonryHeight<Quotient>(u, v, f.material) * freqWeight<Quotient>(t * cone, 40.0f);
+        t = initial + Quotient::div(disp, denom);
       }
     }
   }
@@ -89,7 +89,7 @@ static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f
 
 // Nearest positive hit of one feature, kFar if none (geometry.cu:33-91), in two
 // parts: the slab test every feature starts with (`p`, `d` are the ray in the
-// feature's frame and `inv` = invDir(d)), and the rest.
+// feature's frame and `inv` = invDir<Quotient>(d)), and the rest.
 SD Span featureSlab(const Feat& f, f3 p, f3 inv) {
   const f3 h = f.h;
   return (f.shape == 3 || f.shape == 4) ? slabInv(p, inv, mk(-h.x, 0.0f, -h.z), h) : slabInv(p, inv, h * -1.0f, h);
@@ -101,30 +101,30 @@ SD float featureInSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, Span range, floa
   const f3 h = f.h;
   float t = range.lo > 0.001f ? range.lo : range.hi;
   if (shape == 1) {  // ellipsoid
-    f3 a = mk(p.x / h.x, p.y / h.y, p.z / h.z), v = mk(d.x / h.x, d.y / h.y, d.z / h.z);
+    f3 a = mk(Quotient::div(p.x, h.x), Quotient::div(p.y, h.y), Quotient::div(p.z, h.z)), v = mk(Quotient::div(d.x, h.x), Quotient::div(d.y, h.y), Quotient::div(d.z, h.z));
     float aa = dot(v, v), bb = dot(a, v), cc = dot(a, a) - 1.0f, disc = bb * bb - aa * cc;
     if (disc < 0.0f) return kFar;
-    float sq = sqrtf(disc);
-    t = (-bb - sq) / aa;
-    if (t <= 0.001f) t = (-bb + sq) / aa;
+    float sq = Quotient::root(disc);
+    t = Quotient::div(-bb - sq, aa);
+    if (t <= 0.001f) t = Quotient::div(-bb + sq, aa);
     if (f.material == 7 && t < kFar) t = foliageHit(ro, rd, f.p, h, int(f.seed), range.lo, range.hi);
   } else if (shape == 2) {  // capped vertical cylinder
     const float hx2 = h.x * h.x, hz2 = h.z * h.z;
-    float a = d.x * d.x / hx2 + d.z * d.z / hz2;
-    float bb = p.x * d.x / hx2 + p.z * d.z / hz2;
-    float cc = p.x * p.x / hx2 + p.z * p.z / hz2 - 1.0f;
+    float a = Quotient::div(d.x * d.x, hx2) + Quotient::div(d.z * d.z, hz2);
+    float bb = Quotient::div(p.x * d.x, hx2) + Quotient::div(p.z * d.z, hz2);
+    float cc = Quotient::div(p.x * p.x, hx2) + Quotient::div(p.z * p.z, hz2) - 1.0f;
     float best = kFar, disc = bb * bb - a * cc;
     if (disc >= 0.0f && a > 0.0000001f) {
-      float sq = sqrtf(disc);
-      float u = (-bb - sq) / a, v = (-bb + sq) / a;
+      float sq = Quotient::root(disc);
+      float u = Quotient::div(-bb - sq, a), v = Quotient::div(-bb + sq, a);
       if (u > 0.001f && fabsf(p.y + d.y * u) <= h.y) best = u;
       if (v > 0.001f && fabsf(p.y + d.y * v) <= h.y) best = fminf(best, v);
     }
     if (fabsf(d.y) > 0.000001f) {
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        float cy = k == 0 ? -h.y : h.y, u = (cy - p.y) / d.y;
-        float xx = (p.x + d.x * u) / h.x, zz = (p.z + d.z * u) / h.z;
+        float cy = k == 0 ? -h.y : h.y, u = Quotient::div(cy - p.y, d.y);
+        float xx = Quotient::div(p.x + d.x * u, h.x), zz = Quotient::div(p.z + d.z * u, h.z);
         if (u > 0.001f && xx * xx + zz * zz <= 1.0f) best = fminf(best, u);
       }
     }
@@ -134,27 +134,27 @@ SD float featureInSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, Span range, floa
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       float sg = k == 0 ? 1.0f : -1.0f;
-      float numer = h.y - (p.y + sg * p.x * h.y / h.x), denom = d.y + sg * d.x * h.y / h.x;
+      float numer = h.y - (p.y + Quotient::div(sg * p.x * h.y, h.x)), denom = d.y + Quotient::div(sg * d.x * h.y, h.x);
       if (fabsf(denom) < 0.000001f) { if (numer < 0.0f) return kFar; }
-      else { float u = numer / denom; if (denom > 0.0f) farT = fminf(farT, u); else nearT = fmaxf(nearT, u); }
+      else { float u = Quotient::div(numer, denom); if (denom > 0.0f) farT = fminf(farT, u); else nearT = fmaxf(nearT, u); }
     }
     if (farT < nearT) return kFar;
     t = nearT;
   } else if (shape == 4 || shape == 7) {  // half arch / full ring, radii 1 and 0.77
     const float hx2 = h.x * h.x, hy2 = h.y * h.y;
     float best = kFar;
-    float a = d.x * d.x / hx2 + d.y * d.y / hy2;
-    float bb = p.x * d.x / hx2 + p.y * d.y / hy2;
-    float pq = p.x * p.x / hx2 + p.y * p.y / hy2;
+    float a = Quotient::div(d.x * d.x, hx2) + Quotient::div(d.y * d.y, hy2);
+    float bb = Quotient::div(p.x * d.x, hx2) + Quotient::div(p.y * d.y, hy2);
+    float pq = Quotient::div(p.x * p.x, hx2) + Quotient::div(p.y * p.y, hy2);
 #pragma unroll
     for (int ring = 0; ring < 2; ring++) {
       float rad = ring == 0 ? 1.0f : 0.77f;
       float cc = pq - rad * rad, disc = bb * bb - a * cc;
       if (disc >= 0.0f && a > 0.000001f) {
-        float sq = sqrtf(disc);
+        float sq = Quotient::root(disc);
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-          float u = (-bb + (k == 0 ? -sq : sq)) / a;
+          float u = Quotient::div(-bb + (k == 0 ? -sq : sq), a);
           if (u > 0.001f && fabsf(p.z + d.z * u) <= h.z && (shape == 7 || p.y + d.y * u >= 0.0f)) best = fminf(best, u);
         }
       }
@@ -162,8 +162,8 @@ SD float featureInSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, Span range, floa
     if (fabsf(d.z) > 0.000001f) {
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        float u = ((k == 0 ? -h.z : h.z) - p.z) / d.z;
-        float xx = (p.x + d.x * u) / h.x, yy = (p.y + d.y * u) / h.y, rr = xx * xx + yy * yy;
+        float u = Quotient::div((k == 0 ? -h.z : h.z) - p.z, d.z);
+        float xx = Quotient::div(p.x + d.x * u, h.x), yy = Quotient::div(p.y + d.y * u, h.y), rr = xx * xx + yy * yy;
         if (u > 0.001f && rr <= 1.0f && rr >= 0.77f * 0.77f && (shape == 7 || yy >= 0.0f)) best = fminf(best, u);
       }
     }
@@ -175,7 +175,7 @@ SD float featureInSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, Span range, floa
 }
 SD float featureHit(const Feat& f, f3 ro, f3 rd, float cone) {
   const f3 d = intoFeature(rd, f.turn), p = intoFeature(ro - f.p, f.turn);
-  const Span range = featureSlab(f, p, invDir(d));
+  const Span range = featureSlab(f, p, invDir<Quotient>(d));
   return featureSlabMiss(f, range) ? kFar : featureInSlab(f, ro, rd, p, d, range, cone);
 }
 
@@ -215,21 +215,21 @@ static __device__ __noinline__ f3 featureNormal(Feat f, f3 point) {
   const f3 p = intoFeature(point - f.p, turn), h = f.h;
   f3 n = mk(0.0f, 1.0f, 0.0f);
   if (shape == 1 && f.material == 7)
-    return leafNormal(int(floorf(point.x / 0.18f)), int(floorf(point.y / 0.18f)), int(floorf(point.z / 0.18f)), int(f.seed));
-  if (shape == 1) n = unit(mk(p.x / (h.x * h.x), p.y / (h.y * h.y), p.z / (h.z * h.z)));
+    return leafNormal(int(floorf(Quotient::div(point.x, 0.18f))), int(floorf(Quotient::div(point.y, 0.18f))), int(floorf(Quotient::div(point.z, 0.18f))), int(f.seed));
+  if (shape == 1) n = Quotient::unit(mk(Quotient::div(p.x, h.x * h.x), Quotient::div(p.y, h.y * h.y), Quotient::div(p.z, h.z * h.z)));
   else if (shape == 2) {
     if (fabsf(fabsf(p.y) - h.y) < 0.01f) n = mk(0.0f, p.y < 0.0f ? -1.0f : 1.0f, 0.0f);
-    else n = unit(mk(p.x / (h.x * h.x), 0.0f, p.z / (h.z * h.z)));
+    else n = Quotient::unit(mk(Quotient::div(p.x, h.x * h.x), 0.0f, Quotient::div(p.z, h.z * h.z)));
   } else if (shape == 4 || shape == 7) {
     if (fabsf(fabsf(p.z) - h.z) < 0.008f) n = mk(0.0f, 0.0f, p.z < 0.0f ? -1.0f : 1.0f);
     else {
-      float rr = p.x * p.x / (h.x * h.x) + p.y * p.y / (h.y * h.y);
-      n = unit(mk(p.x / (h.x * h.x), p.y / (h.y * h.y), 0.0f)) * (rr < 0.8f ? -1.0f : 1.0f);
+      float rr = Quotient::div(p.x * p.x, h.x * h.x) + Quotient::div(p.y * p.y, h.y * h.y);
+      n = Quotient::unit(mk(Quotient::div(p.x, h.x * h.x), Quotient::div(p.y, h.y * h.y), 0.0f)) * (rr < 0.8f ? -1.0f : 1.0f);
     }
   } else if (shape == 3) {
     if (fabsf(fabsf(p.z) - h.z) < 0.006f) n = mk(0.0f, 0.0f, p.z < 0.0f ? -1.0f : 1.0f);
     else if (p.y < 0.003f) n = mk(0.0f, -1.0f, 0.0f);
-    else n = unit(mk(p.x < 0.0f ? -h.y / h.x : h.y / h.x, 1.0f, 0.0f));
+    else n = Quotient::unit(mk(Quotient::div(p.x < 0.0f ? -h.y : h.y, h.x), 1.0f, 0.0f));
   } else {
     f3 a = mk(fabsf(fabsf(p.x) - h.x), fabsf(fabsf(p.y) - h.y), fabsf(fabsf(p.z) - h.z));
     n = a.x < a.y && a.x < a.z ? mk(p.x < 0.0f ? -1.0f : 1.0f, 0.0f, 0.0f)
@@ -238,7 +238,7 @@ static __device__ __noinline__ f3 featureNormal(Feat f, f3 point) {
     f3 q = mk(fmaxf(fabsf(p.x) - h.x + bevel, 0.0f) * (p.x < 0.0f ? -1.0f : 1.0f),
               fmaxf(fabsf(p.y) - h.y + bevel, 0.0f) * (p.y < 0.0f ? -1.0f : 1.0f),
               fmaxf(fabsf(p.z) - h.z + bevel, 0.0f) * (p.z < 0.0f ? -1.0f : 1.0f));
-    if (dot(q, q) > 0.000001f) n = unit(q);
+    if (dot(q, q) > 0.000001f) n = Quotient::unit(q);
   }
   return outOfFeature(n, turn);
 }

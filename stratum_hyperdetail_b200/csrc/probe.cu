@@ -1,5 +1,6 @@
 // probeGrammar (kernels/probe.cu:2-14 of the reference) and the grammar
 // enumeration service: feature records of many (lot, group) pairs in one launch.
+#define STRATUM_QUOTIENT WrittenOut
 #include "common_api.cuh"
 #include "geometry.cuh"
 

@@ -11,6 +11,9 @@
 // (distance, index) in whatever order the features are tested.
 #include <mutex>
 
+// (written out: the features of one ray keep coming back to the same code; with one
+// copy of each 65,536 rays take 0.62 ms instead of 0.47)
+#define STRATUM_QUOTIENT WrittenOut
 #include "common_api.cuh"
 #include "grammar_ra.cuh"
 #include "traverse.cuh"

@@ -57,8 +57,35 @@ HD float clampv(float x, float a, float b) { return fminf(b, fmaxf(a, x)); }
 HD float sat(float x) { return clampv(x, 0.0f, 1.0f); }
 HD float lerp(float a, float b, float t) { return a + (b - a) * t; }
 HD float fract(float x) { return x - floorf(x); }
-HD float smooth(float a, float b, float x) {
-  float t = sat((x - a) / (b - a));
+// ---- divisions and square roots ----------------------------------------------
+// An IEEE division or square root takes 8-10 instructions and a branch where it is
+// written out.  The trace kernels run once through most of their code for each tile and
+// wait for instructions first of all, so they call one copy (OneCopy: 108 KB of
+// code to 90, six-view 1600x900 trace 4.62 -> 4.34 ms); shading loops over the same
+// code tile after tile and is faster with them written out (392 against 427 us for
+// the material pass).  Same results.
+struct WrittenOut {
+  static HD float div(float a, float b) { return a / b; }
+  static HD float root(float a) { return sqrtf(a); }
+  static HD f3 unit(f3 a) { return st::unit(a); }
+};
+static __device__ __noinline__ float divideOnce(float a, float b) { return a / b; }
+static __device__ __noinline__ float rootOnce(float a) { return sqrtf(a); }
+static __device__ __noinline__ f3 unitOnce(f3 a) { return unit(a); }
+struct OneCopy {
+  static SD float div(float a, float b) { return divideOnce(a, b); }
+  static SD float root(float a) { return rootOnce(a); }
+  static SD f3 unit(f3 a) { return unitOnce(a); }
+};
+// How a file's kernels divide in the code they share (a file defines
+// STRATUM_QUOTIENT before its includes to choose otherwise).
+#ifndef STRATUM_QUOTIENT
+#define STRATUM_QUOTIENT OneCopy
+#endif
+using Quotient = STRATUM_QUOTIENT;
+
+template <class Q = WrittenOut> HD float smooth(float a, float b, float x) {
+  float t = sat(Q::div(x - a, b - a));
   return t * t * (3.0f - 2.0f * t);
 }
 HD int imod(int x, int n) { int r = x % n; return r < 0 ? r + n : r; }
@@ -95,7 +122,9 @@ HD float fbm2(float x, float y) {
   }
   return v;
 }
-HD float freqWeight(float footprint, float freq) { return 1.0f - smooth(0.35f, 1.1f, footprint * freq); }
+template <class Q = WrittenOut> HD float freqWeight(float footprint, float freq) {
+  return 1.0f - smooth<Q>(0.35f, 1.1f, footprint * freq);
+}
 
 // ---- camera (common.cu:54-70) -----------------------------------------------
 // sin/cos of the camera angles in double, rounded once to float.
@@ -126,10 +155,10 @@ HD Camera makeCamera(const float* C) {
   if (sample > 0) { c.jx = halton(sample, 2) - 0.5f; c.jy = halton(sample, 3) - 0.5f; }
   return c;
 }
-HD f3 primaryDir(const Camera& c, int x, int y, int width, int height) {
-  float sx = (float(x) + 0.5f + c.jx - float(width) * 0.5f) / float(height) * 1.08f;
-  float sy = -(float(y) + 0.5f + c.jy - float(height) * 0.5f) / float(height) * 1.08f;
-  return unit(c.fwd + c.right * sx + c.up * sy);
+template <class Q = WrittenOut> HD f3 primaryDir(const Camera& c, int x, int y, int width, int height) {
+  float sx = Q::div(float(x) + 0.5f + c.jx - float(width) * 0.5f, float(height)) * 1.08f;
+  float sy = Q::div(-(float(y) + 0.5f + c.jy - float(height) * 0.5f), float(height)) * 1.08f;
+  return Q::unit(c.fwd + c.right * sx + c.up * sy);
 }
 HD f3 sunDir(const float* C) {
   float s7 = sinR(C[7]), c7 = cosR(C[7]), s8 = sinR(C[8]), c8 = cosR(C[8]);
@@ -137,8 +166,8 @@ HD f3 sunDir(const float* C) {
 }
 
 // ---- slab test (common.cu:71-77) --------------------------------------------
-HD float guardedInv(float d) {
-  return 1.0f / (fabsf(d) > 0.0000001f ? d : (d < 0.0f ? -0.0000001f : 0.0000001f));
+template <class Q = WrittenOut> HD float guardedInv(float d) {
+  return Q::div(1.0f, fabsf(d) > 0.0000001f ? d : (d < 0.0f ? -0.0000001f : 0.0000001f));
 }
 struct Span { float lo, hi; };
 HD Span slabInv(f3 ro, f3 inv, f3 lo, f3 hi) {
@@ -147,7 +176,9 @@ HD Span slabInv(f3 ro, f3 inv, f3 lo, f3 hi) {
   f3 mn = vmin(a, b), mx = vmax(a, b);
   return {fmaxf(fmaxf(mn.x, mn.y), mn.z), fminf(fminf(mx.x, mx.y), mx.z)};
 }
-HD f3 invDir(f3 rd) { return mk(guardedInv(rd.x), guardedInv(rd.y), guardedInv(rd.z)); }
+template <class Q = WrittenOut> HD f3 invDir(f3 rd) {
+  return mk(guardedInv<Q>(rd.x), guardedInv<Q>(rd.y), guardedInv<Q>(rd.z));
+}
 HD Span slab(f3 ro, f3 rd, f3 lo, f3 hi) { return slabInv(ro, invDir(rd), lo, hi); }
 
 // ---- masonry relief (common.cu:78-87) ---------------------------------------
@@ -156,10 +187,11 @@ HD void masonryUV(f3 p, f3 n, float& u, float& v) {
   else if (fabsf(n.x) > 0.5f) { u = p.z; v = p.y; }
   else { u = p.x; v = p.y; }
 }
-HD float masonryHeight(float u, float v, int material) {
+template <class Q = WrittenOut> HD float masonryHeight(float u, float v, int material) {
   float bw = material == 1 ? 0.46f : 0.92f, bh = material == 1 ? 0.215f : 0.46f;
-  int row = int(floorf(v / bh));
-  float x = fract(u / bw + float(imod(row, 2)) * 0.5f), y = fract(v / bh);
+  const float vb = Q::div(v, bh);
+  int row = int(floorf(vb));
+  float x = fract(Q::div(u, bw) + float(imod(row, 2)) * 0.5f), y = fract(vb);
   float edge = fminf(fminf(x, 1.0f - x) * bw, fminf(y, 1.0f - y) * bh);
   float grain = noise2(u * 24.0f, v * 24.0f);
   // The chipping noise takes up to 0.006 m off the edge distance before the step
@@ -169,8 +201,8 @@ HD float masonryHeight(float u, float v, int material) {
   if (edge > 0.008f) {
     mortar = 0.0f;
     if (!(edge - 0.006f >= 0.023f)) {
-      float chipped = edge - 0.006f * smooth(0.34f, 0.73f, noise2(u * 117.0f, v * 117.0f));
-      mortar = 1.0f - smooth(0.008f, 0.023f, chipped);
+      float chipped = edge - 0.006f * smooth<Q>(0.34f, 0.73f, noise2(u * 117.0f, v * 117.0f));
+      mortar = 1.0f - smooth<Q>(0.008f, 0.023f, chipped);
     }
   }
   return -0.018f * mortar + 0.0025f * grain;

@@ -22,6 +22,9 @@
 // safe only when the preceding kernel is known to be another strip.
 #include <mutex>
 
+// (written out: six 3840x2160 views 23.7 ms in one call each, with one copy of each
+// division 24.7; blocks of eight warps here share more of their way through the code)
+#define STRATUM_QUOTIENT WrittenOut
 #include "batch.cuh"
 #include "common_api.cuh"
 #include "traverse_coop.cuh"
@@ -88,7 +91,7 @@ __global__ void __launch_bounds__(kDropInThreads, STRATUM_DROPIN_BLOCKS)
   }
   const bool active = mine && x < width && y < strip;
   y += rowStart;
-  const f3 rd = primaryDir(cam, active ? x : 0, active ? y : 0, width, height);
+  const f3 rd = primaryDir<Quotient>(cam, active ? x : 0, active ? y : 0, width, height);
   const TraceResult r = traceWarp<true>(W, reinterpret_cast<const float4*>(N), org[0], org[2], cam.pos, rd,
                                         1.08f / float(height), active, sh.stage[warp], groupCache(nullptr),
                                         &sh.cache);

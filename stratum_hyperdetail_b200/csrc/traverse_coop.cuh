@@ -20,9 +20,11 @@
 //    intersection routine;
 //  * the winner's normal, material and seed are recomputed once per ray.
 //
-// What bounds the kernel is instruction issue and latency, and code size beyond
-// the instruction cache (108 KB here; at 150 KB the aerial pose took twice as long
-// on instruction fetch).  Six-view 1600x900 trace: each ray walking all records of
+// What bounds the kernel is waiting for instructions (4 of the 9 cycles a warp waits
+// per issue: a tile runs once through most of its 87 KB of code), then dependent
+// arithmetic and loads.  One copy of each division, square root and of the step to
+// the next leaf took the six-view trace from 4.62 to 4.23 ms at 108 -> 87 KB; at 150 KB
+// the aerial pose took twice as long.  Six-view 1600x900 trace: each ray walking all records of
 // a group behind a box test per run of four, 1,000 (aerial) to 2,500 (street)
 // instructions an evaluation, 7.61 ms; records by packet 6.80 ms; without the
 // arithmetic of masonry relief and prisms that is certain to come to nothing
@@ -135,7 +137,7 @@ SD bool packetMayHit(const StagedFeat& s, const Packet& k) {
          (in <= k.best || !(shape == 0 || shape == 3));
 }
 
-enum LaneState : int { kEnterLot = 0, kLotPending = 1, kLeafPending = 2, kDone = 3 };
+enum LaneState : int { kEnterLot = 0, kLotPending = 1, kLeafPending = 2, kDone = 3, kNextLeaf = 4 };
 
 struct CoopRay {
   // ray and result
@@ -166,12 +168,12 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   r.ddaSteps = 0;
   if (!active) return;
   if (rd.y < -0.000001f) {
-    float ground = -ro.y / rd.y;
+    float ground = Quotient::div(-ro.y, rd.y);
     if (ground > 0.001f && ground < r.best) { r.best = ground; r.fid = kGroundId; }
   }
   float nearT = 0.001f, farT = r.best;
   if (fabsf(rd.y) > 0.0000001f) {
-    float a = (-0.5f - ro.y) / rd.y, c = (kTop - ro.y) / rd.y;
+    float a = Quotient::div(-0.5f - ro.y, rd.y), c = Quotient::div(kTop - ro.y, rd.y);
     nearT = fmaxf(nearT, fminf(a, c));
     farT = fminf(farT, fmaxf(a, c));
   } else if (ro.y > kTop || ro.y < -0.5f) farT = -1.0f;
@@ -179,11 +181,11 @@ SD void coopBegin(CoopRay& r, f3 ro, f3 rd, float cone, bool active) {
   if (!(nearT <= farT)) { r.state = kDone; return; }
   r.t = nearT + 0.0002f;
   f3 start = ro + rd * r.t;
-  r.cx = int(floorf((start.x + 18.0f) / kCell));
-  r.cz = int(floorf((start.z + 18.0f) / kCell));
+  r.cx = int(floorf(Quotient::div(start.x + 18.0f, kCell)));
+  r.cz = int(floorf(Quotient::div(start.z + 18.0f, kCell)));
   r.sx = rd.x > 0.0f ? 1 : -1;
   r.sz = rd.z > 0.0f ? 1 : -1;
-  r.inv = invDir(rd);
+  r.inv = invDir<Quotient>(rd);
   r.tx = (float(r.cx) * kCell + (r.sx > 0 ? 18.0f : -18.0f) - ro.x) * r.inv.x;
   r.tz = (float(r.cz) * kCell + (r.sz > 0 ? 18.0f : -18.0f) - ro.z) * r.inv.z;
 }
@@ -275,7 +277,7 @@ SD Packet lotPacket(const CoopRay& r, bool peer, int src) {
 // with one sign flipped, except for an exactly zero ld.x, whose guarded inverse
 // keeps the sign of the zero.
 SD f3 inv1Of(const CoopRay& r) {
-  return mk(r.inv0.z, r.inv0.y, r.ld.x == 0.0f ? guardedInv(-r.ld.x) : -r.inv0.x);
+  return mk(r.inv0.z, r.inv0.y, r.ld.x == 0.0f ? guardedInv<Quotient>(-r.ld.x) : -r.inv0.x);
 }
 
 // The winner's record for one lane: from the group cache when it holds the
@@ -477,44 +479,44 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
   return count;
 }
 
+// Find and order the leaves of every lane in `lots` (lanes that wait in a lot).  Warp-collective.
+SD void coopLots(CoopRay& r, const float4* __restrict__ N, unsigned lots) {
+  const int lane = int(threadIdx.x & 31);
+#pragma unroll 1
+  while (lots) {
+    const int src = __ffs(lots) - 1, slot = __shfl_sync(0xffffffffu, r.slot, src);
+    const bool peer = r.state == kLotPending && r.slot == slot;
+    lots &= ~__ballot_sync(0xffffffffu, peer);
+    // lanes are leaves: which of the lot's 64 can any peer's ray enter
+    const float4* leaf = N + 2 * (slot * kNodes + kGroups + lane);
+    const float4 a0 = __ldg(leaf), b0 = __ldg(leaf + 1), a1 = __ldg(leaf + 64), b1 = __ldg(leaf + 65);
+    const Packet pk = lotPacket(r, peer, src);
+    const unsigned m0 = __ballot_sync(0xffffffffu, a0.w > 0.5f && packetMayEnter(a0, b0, pk));
+    const unsigned m1 = __ballot_sync(0xffffffffu, a1.w > 0.5f && packetMayEnter(a1, b1, pk));
+    if (peer) {
+      const int base = slot * kNodes + kGroups;
+      r.leaves = 0ull;
+#pragma unroll 1
+      for (unsigned long long rest = (unsigned long long)m1 << 32 | m0; rest; rest &= rest - 1ull) {
+        const int k = __ffsll(rest) - 1;
+        if (nodeEntry(N, base + k, r.lr, r.inv0, r.best) < r.best) r.leaves |= 1ull << k;
+      }
+      orderLeaves(r, N);
+      r.state = kNextLeaf;
+    }
+    __syncwarp();
+  }
+}
+
 // Advance every lane until it has a leaf to evaluate or is done.  Warp-collective.
 SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __restrict__ N, uint32_t o0, uint32_t o2) {
-  const int lane = int(threadIdx.x & 31);
 #pragma unroll 1
   for (;;) {
     coopEnterLot(r, W, N, o0, o2);
-    unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
+    const unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
     if (!lots) return;
-#pragma unroll 1
-    while (lots) {
-      const int src = __ffs(lots) - 1, slot = __shfl_sync(0xffffffffu, r.slot, src);
-      const bool peer = r.state == kLotPending && r.slot == slot;
-      lots &= ~__ballot_sync(0xffffffffu, peer);
-      // lanes are leaves: which of the lot's 64 can any peer's ray enter
-      const float4* leaf = N + 2 * (slot * kNodes + kGroups + lane);
-      const float4 a0 = __ldg(leaf), b0 = __ldg(leaf + 1), a1 = __ldg(leaf + 64), b1 = __ldg(leaf + 65);
-      const Packet pk = lotPacket(r, peer, src);
-      unsigned m0 = __ballot_sync(0xffffffffu, a0.w > 0.5f && packetMayEnter(a0, b0, pk));
-      unsigned m1 = __ballot_sync(0xffffffffu, a1.w > 0.5f && packetMayEnter(a1, b1, pk));
-      if (peer) {
-        const int base = slot * kNodes + kGroups;
-        unsigned lo = 0u, hi = 0u;
-#pragma unroll 1
-        for (; m0; m0 &= m0 - 1u) {
-          const int k = __ffs(m0) - 1;
-          if (nodeEntry(N, base + k, r.lr, r.inv0, r.best) < r.best) lo |= 1u << k;
-        }
-#pragma unroll 1
-        for (; m1; m1 &= m1 - 1u) {
-          const int k = __ffs(m1) - 1;
-          if (nodeEntry(N, base + 32 + k, r.lr, r.inv0, r.best) < r.best) hi |= 1u << k;
-        }
-        r.leaves = (unsigned long long)hi << 32 | lo;
-        orderLeaves(r, N);
-        nextLeaf(r, N);
-      }
-      __syncwarp();
-    }
+    coopLots(r, N, lots);
+    if (r.state == kNextLeaf) nextLeaf(r, N);
   }
 }
 
@@ -530,65 +532,79 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
   const int lane = int(threadIdx.x & 31);
   CoopRay r;
   coopBegin(r, ro, rd, cone, active);
+  bool advancing = true;  // until every lane waits on a leaf or is done; then all their leaves are served
 #pragma unroll 1
   for (;;) {
-    coopAdvance(r, W, N, o0, o2);
-    unsigned pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
-    if (!pending) break;  // every lane is done (lanes only stop advancing at a leaf or when done)
-#pragma unroll 1
-    while (pending) {
-      // the first pending lane's (lot, group), for every lane that waits on it
-      const int myKey = (r.slot << 6) | r.pend;
-      const int key = __shfl_sync(0xffffffffu, myKey, __ffs(pending) - 1);
-      const bool peer = r.state == kLeafPending && myKey == key;
-      const unsigned peers = __ballot_sync(0xffffffffu, peer);
-      // lanes are records: which of the group's can any peer's ray hit
-      StagedFeat r0, r1;
-      const int count = groupRecords<kBlockCache>(W, cache, bc, key, ws, r0, r1);
-      const Packet pk = lotPacket(r, peer, __ffs(peers) - 1);
-      const unsigned m0 = __ballot_sync(0xffffffffu, lane < count && packetMayHit(r0, pk));
-      const unsigned m1 = count <= 32 ? 0u : __ballot_sync(0xffffffffu, lane + 32 < count && packetMayHit(r1, pk));
-      if ((m0 >> lane) & 1u) ws.feats[lane] = r0;
-      if ((m1 >> lane) & 1u) ws.feats[lane + 32] = r1;
-      __syncwarp();
-      if (peer) {
-        // those records in index order: the first feature wins ties
-        const int g = r.pend;
-        unsigned mlo = m0, mhi = m1;
-#pragma unroll 1
-        while (mlo | mhi) {
-          const int k = mlo ? __ffs(mlo) - 1 : __ffs(mhi) + 31;
-          if (mlo) mlo &= mlo - 1u; else mhi &= mhi - 1u;
-          const Feat f = unstage(ws.feats[k]);
-          const bool odd = f.turn % 2 == 1;
-          const f3 inv = odd ? inv1Of(r) : r.inv0, p = intoFeature(r.lr - f.p, f.turn);
-          const Span rg = featureSlab(f, p, inv);
-          if (featureSlabMiss(f, rg)) continue;
-          float th;
-          if (plainBox(f)) {
-            th = plainBoxHit(rg);
-          } else {
-            const f3 d = odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld;
-            if (f.shape == 3) {  // its distance is never before the slab's entry
-              if (rg.lo > r.best || prismMiss(f, p, d, rg)) continue;
-            } else {
-              f3 lo, hi;
-              hitBox(f, lo, hi);
-              const Span cr = slabInv(r.lr, r.inv0, lo, hi);
-              if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
-            }
-            th = featureInSlabOOL(f, r.lr, r.ld, p, d, rg, r.cone);
-          }
-          if (th > 0.001f && th < r.best) {
-            r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
-            r.moved = true;
-          }
-        }
-        nextLeaf(r, N);
+    if (r.state == kNextLeaf) nextLeaf(r, N);
+    if (advancing) {
+      coopEnterLot(r, W, N, o0, o2);
+      const unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
+      if (lots) {
+        coopLots(r, N, lots);
+        continue;
       }
-      __syncwarp();
-      pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
     }
+    const unsigned pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
+    if (!pending) {
+      if (advancing) break;  // every lane is done
+      advancing = true;
+      continue;
+    }
+    advancing = false;
+    // the first pending lane's (lot, group), for every lane that waits on it
+    const int myKey = (r.slot << 6) | r.pend;
+    const int key = __shfl_sync(0xffffffffu, myKey, __ffs(pending) - 1);
+    const bool peer = r.state == kLeafPending && myKey == key;
+    const unsigned peers = __ballot_sync(0xffffffffu, peer);
+    // lanes are records: which of the group's can any peer's ray hit
+    StagedFeat r0, r1;
+    const int count = groupRecords<kBlockCache>(W, cache, bc, key, ws, r0, r1);
+    const Packet pk = lotPacket(r, peer, __ffs(peers) - 1);
+    unsigned m0 = 0u, m1 = 0u;
+#pragma unroll 1
+    for (int half = 0; half < count; half += 32) {
+      if (half) r0 = r1;
+      const unsigned m = __ballot_sync(0xffffffffu, lane + half < count && packetMayHit(r0, pk));
+      if ((m >> lane) & 1u) ws.feats[lane + half] = r0;
+      if (half) m1 = m; else m0 = m;
+    }
+    __syncwarp();
+    if (peer) {
+      // those records in index order: the first feature wins ties
+      const int g = r.pend;
+      unsigned mlo = m0, mhi = m1;
+#pragma unroll 1
+      while (mlo | mhi) {
+        const int k = mlo ? __ffs(mlo) - 1 : __ffs(mhi) + 31;
+        if (mlo) mlo &= mlo - 1u; else mhi &= mhi - 1u;
+        const Feat f = unstage(ws.feats[k]);
+        const bool odd = f.turn % 2 == 1;
+        const f3 inv = odd ? inv1Of(r) : r.inv0, p = intoFeature(r.lr - f.p, f.turn);
+        const Span rg = featureSlab(f, p, inv);
+        if (featureSlabMiss(f, rg)) continue;
+        float th;
+        if (plainBox(f)) {
+          th = plainBoxHit(rg);
+        } else {
+          const f3 d = odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld;
+          if (f.shape == 3) {  // its distance is never before the slab's entry
+            if (rg.lo > r.best || prismMiss(f, p, d, rg)) continue;
+          } else {
+            f3 lo, hi;
+            hitBox(f, lo, hi);
+            const Span cr = slabInv(r.lr, r.inv0, lo, hi);
+            if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
+          }
+          th = featureInSlabOOL(f, r.lr, r.ld, p, d, rg, r.cone);
+        }
+        if (th > 0.001f && th < r.best) {
+          r.best = th; r.fid = g * kMaxFeatures + k; r.wslot = r.slot; r.wcx = r.lcx; r.wcz = r.lcz;
+          r.moved = true;
+        }
+      }
+      r.state = kNextLeaf;
+    }
+    __syncwarp();
   }
   TraceResult out;
   out.t = r.best; out.fid = r.fid; out.material = 10; out.seed = 0.0f; out.slot = -1;
