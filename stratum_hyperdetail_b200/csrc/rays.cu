@@ -208,6 +208,10 @@ __global__ void __launch_bounds__(64) traceRaysK(const float* __restrict__ W, co
 // rays of a block in length.  8,192 random rays: a thread per ray (256 warps for
 // 592 schedulers, 1,859 features a lot one after another) 59 ms; one lot of eight rays at
 // a time with four groups across the lanes 6.0 ms (6.6 of 32 lanes active).
+// Rays differ several times over in the lots they cross, so no slot is given rays
+// of its own: the block's next ray goes to whichever slot is free.  2,000 rays take
+// 1.43 ms and 8,192 2.29 (fixed slots 2.55 and 3.5; a contiguous run of the rays to a
+// block, whose neighbours are alike, 1.98 and 7.2).
 constexpr int kExRays = 8, kExLots = 4, kExWarps = 16;
 // Group k of a warp's four.
 SD int warpGroup(int w, int k) {
@@ -230,7 +234,7 @@ struct NearestSink {
     if (th > 0.001f && th < t) { t = th; id = k; }
   }
 };
-// (128 registers: at 64, two blocks an SM, 6.3 ms against 3.6)
+// (128 registers: at 64, two blocks an SM, 6.3 ms against 3.6 with fixed slots)
 __global__ void __launch_bounds__(32 * kExWarps, 1)
     traceExhaustiveK(const float* __restrict__ W, const uint32_t* __restrict__ O, const float* __restrict__ rays, int n,
                      float* out) {
@@ -242,15 +246,20 @@ __global__ void __launch_bounds__(32 * kExWarps, 1)
   const uint32_t o0 = O[0], o2 = O[2];
   if (threadIdx.x < 96) least[threadIdx.x / 32][threadIdx.x % 32] = none;
   __syncthreads();
-  unsigned i = blockIdx.x * kExRays + unsigned(mine);
-  const unsigned stride = gridDim.x * kExRays, end = unsigned(n);
+  // the block's rays are blockIdx.x, blockIdx.x + gridDim.x, ...; a slot that has
+  // finished its own takes the next of them
+  const unsigned share = (unsigned(n) - blockIdx.x + gridDim.x - 1u) / gridDim.x;
+  unsigned next = 0u, i = 0u;
   int turn = 0;
   bool begun = false;
   RayDda r;  // before the next four lots; the same on every lane of the ray in every warp
 #pragma unroll 1
   for (;;) {
-    if (!begun && i < end) {
-      if (!ddaBegin(r, rays + size_t(i) * 7)) r.steps = 160;  // nothing to visit
+    const unsigned idle = __ballot_sync(0xffffffffu, !begun) & ((1u << kExRays) - 1u);
+    if (!begun) i = next + __popc(idle & ((1u << mine) - 1u));
+    next += __popc(idle);
+    if (!begun && i < share) {
+      if (!ddaBegin(r, rays + (size_t(i) * gridDim.x + blockIdx.x) * 7)) r.steps = 160;  // nothing to visit
       begun = true;
     }
     if (!__any_sync(0xffffffffu, begun)) break;  // every warp holds the same rays: uniform over the block
@@ -277,8 +286,8 @@ __global__ void __launch_bounds__(32 * kExWarps, 1)
       }
       if (key != none) atomicMin(&least[turn][lane], key);
     }
-    const int next = turn == 2 ? 0 : turn + 1;
-    if (threadIdx.x < 32) least[next][threadIdx.x] = none;
+    const int after = turn == 2 ? 0 : turn + 1;
+    if (threadIdx.x < 32) least[after][threadIdx.x] = none;
     __syncthreads();
     if (begun) {
       bool open = true;
@@ -297,12 +306,11 @@ __global__ void __launch_bounds__(32 * kExWarps, 1)
         ddaStep(r);
       }
       if (!open) {
-        if (warp == 0 && ahead == 0) ddaStore(r, W, out + size_t(i) * 8);
-        i = end - i > stride ? i + stride : end;
+        if (warp == 0 && ahead == 0) ddaStore(r, W, out + (size_t(i) * gridDim.x + blockIdx.x) * 8);
         begun = false;
       }
     }
-    turn = next;
+    turn = after;
   }
 }
 
