@@ -4,13 +4,18 @@
 // results bit for bit, organised for a warp of 32 coherent rays (one 8x4 tile):
 //
 //  * each lane steps its own lot DDA to the next lot whose root it enters;
-//  * the warp takes the lots its lanes wait in one at a time.  Lanes stand for
-//    leaves: all 64 groups of the lot are tested at once against the waiting rays,
-//    taken as a packet (packetMayEnter), and each ray then tests the few leaves
-//    left (3-6) itself and orders its own by the reference's near-first descent,
+//  * the warp takes the lots its lanes wait in one at a time, the one fewest cells
+//    from the camera's first: a ray that reaches a lot has come through nearer
+//    ones, so each lot is met once with every ray that will enter it (all lanes'
+//    next lots in turn, whatever their distance: 3.88 ms against 3.45, below).  Lanes
+//    stand for leaves: all 64 groups of the lot are tested at once against the
+//    waiting rays, taken as a packet (packetMayEnter), and each ray then tests the few
+//    leaves left (3-6) itself and orders its own by the reference's near-first descent,
 //    which needs the hierarchy only where the paths to two of its leaves part;
-//  * when every lane waits on a leaf or is done, the warp evaluates one distinct
-//    (lot, group) at a time for all the lanes that wait on it.  Its records come
+//  * the warp evaluates one group of that lot at a time for all the lanes that wait
+//    on it, the one whose ray has the most leaves to go first, since a ray that is
+//    behind may yet come to a group others wait on (the first lane's group instead
+//    4.14 ms against 3.88, the nearest 4.34).  Its records come
 //    from the table's group cache (group_cache.cuh), the block's table (the
 //    drop-in), or the random-access grammar (grammar_ra.cuh), which stores them
 //    when the cache has room.  Lanes now stand for records and test them against
@@ -23,8 +28,9 @@
 // What bounds the kernel is waiting for instructions (4 of the 9 cycles a warp waits
 // per issue: a tile runs once through most of its 87 KB of code), then dependent
 // arithmetic and loads.  One copy of each division, square root and of the step to
-// the next leaf took the six-view trace from 4.62 to 4.23 ms at 108 -> 87 KB; at 150 KB
-// the aerial pose took twice as long.  Six-view 1600x900 trace: each ray walking all records of
+// the next leaf took the six-view trace from 4.62 to 4.14 ms at 108 -> 87 KB; at 150 KB
+// the aerial pose took twice as long.  Lots and groups in the order above: 3.45 ms
+// (street 0.61 -> 0.43, aerial 1.89 -> 1.54).  Six-view 1600x900 trace: each ray walking all records of
 // a group behind a box test per run of four, 1,000 (aerial) to 2,500 (street)
 // instructions an evaluation, 7.61 ms; records by packet 6.80 ms; without the
 // arithmetic of masonry relief and prisms that is certain to come to nothing
@@ -479,33 +485,28 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
   return count;
 }
 
-// Find and order the leaves of every lane in `lots` (lanes that wait in a lot).  Warp-collective.
-SD void coopLots(CoopRay& r, const float4* __restrict__ N, unsigned lots) {
-  const int lane = int(threadIdx.x & 31);
+// Find and order the leaves of every lane that waits in lane `src`'s lot; those lanes.  Warp-collective.
+SD unsigned coopLot(CoopRay& r, const float4* __restrict__ N, int src) {
+  const int lane = int(threadIdx.x & 31), slot = __shfl_sync(0xffffffffu, r.slot, src);
+  const bool peer = r.state == kLotPending && r.slot == slot;
+  // lanes are leaves: which of the lot's 64 can any peer's ray enter
+  const float4* leaf = N + 2 * (slot * kNodes + kGroups + lane);
+  const float4 a0 = __ldg(leaf), b0 = __ldg(leaf + 1), a1 = __ldg(leaf + 64), b1 = __ldg(leaf + 65);
+  const Packet pk = lotPacket(r, peer, src);
+  const unsigned m0 = __ballot_sync(0xffffffffu, a0.w > 0.5f && packetMayEnter(a0, b0, pk));
+  const unsigned m1 = __ballot_sync(0xffffffffu, a1.w > 0.5f && packetMayEnter(a1, b1, pk));
+  if (peer) {
+    const int base = slot * kNodes + kGroups;
+    r.leaves = 0ull;
 #pragma unroll 1
-  while (lots) {
-    const int src = __ffs(lots) - 1, slot = __shfl_sync(0xffffffffu, r.slot, src);
-    const bool peer = r.state == kLotPending && r.slot == slot;
-    lots &= ~__ballot_sync(0xffffffffu, peer);
-    // lanes are leaves: which of the lot's 64 can any peer's ray enter
-    const float4* leaf = N + 2 * (slot * kNodes + kGroups + lane);
-    const float4 a0 = __ldg(leaf), b0 = __ldg(leaf + 1), a1 = __ldg(leaf + 64), b1 = __ldg(leaf + 65);
-    const Packet pk = lotPacket(r, peer, src);
-    const unsigned m0 = __ballot_sync(0xffffffffu, a0.w > 0.5f && packetMayEnter(a0, b0, pk));
-    const unsigned m1 = __ballot_sync(0xffffffffu, a1.w > 0.5f && packetMayEnter(a1, b1, pk));
-    if (peer) {
-      const int base = slot * kNodes + kGroups;
-      r.leaves = 0ull;
-#pragma unroll 1
-      for (unsigned long long rest = (unsigned long long)m1 << 32 | m0; rest; rest &= rest - 1ull) {
-        const int k = __ffsll(rest) - 1;
-        if (nodeEntry(N, base + k, r.lr, r.inv0, r.best) < r.best) r.leaves |= 1ull << k;
-      }
-      orderLeaves(r, N);
-      r.state = kNextLeaf;
+    for (unsigned long long rest = (unsigned long long)m1 << 32 | m0; rest; rest &= rest - 1ull) {
+      const int k = __ffsll(rest) - 1;
+      if (nodeEntry(N, base + k, r.lr, r.inv0, r.best) < r.best) r.leaves |= 1ull << k;
     }
-    __syncwarp();
+    orderLeaves(r, N);
+    r.state = kNextLeaf;
   }
+  return __ballot_sync(0xffffffffu, peer);
 }
 
 // Advance every lane until it has a leaf to evaluate or is done.  Warp-collective.
@@ -513,9 +514,10 @@ SD void coopAdvance(CoopRay& r, const float* __restrict__ W, const float4* __res
 #pragma unroll 1
   for (;;) {
     coopEnterLot(r, W, N, o0, o2);
-    const unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
+    unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
     if (!lots) return;
-    coopLots(r, N, lots);
+#pragma unroll 1
+    while (lots) lots &= ~coopLot(r, N, __ffs(lots) - 1);
     if (r.state == kNextLeaf) nextLeaf(r, N);
   }
 }
@@ -532,28 +534,23 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
   const int lane = int(threadIdx.x & 31);
   CoopRay r;
   coopBegin(r, ro, rd, cone, active);
-  bool advancing = true;  // until every lane waits on a leaf or is done; then all their leaves are served
 #pragma unroll 1
   for (;;) {
     if (r.state == kNextLeaf) nextLeaf(r, N);
-    if (advancing) {
+    if (!__any_sync(0xffffffffu, r.state == kLeafPending)) {
       coopEnterLot(r, W, N, o0, o2);
-      const unsigned lots = __ballot_sync(0xffffffffu, r.state == kLotPending);
-      if (lots) {
-        coopLots(r, N, lots);
-        continue;
-      }
-    }
-    const unsigned pending = __ballot_sync(0xffffffffu, r.state == kLeafPending);
-    if (!pending) {
-      if (advancing) break;  // every lane is done
-      advancing = true;
+      // the lot fewest cells away (the camera is in cell 0 or next to it)
+      const unsigned far = r.state == kLotPending ? unsigned(abs(r.lcx) + abs(r.lcz)) : ~0u;
+      const unsigned nearest = __reduce_min_sync(0xffffffffu, far);
+      if (nearest == ~0u) break;  // every lane is done
+      coopLot(r, N, __ffs(__ballot_sync(0xffffffffu, far == nearest)) - 1);
       continue;
     }
-    advancing = false;
-    // the first pending lane's (lot, group), for every lane that waits on it
+    // a lane's group, the one with most leaves to go, for every lane that waits on it
     const int myKey = (r.slot << 6) | r.pend;
-    const int key = __shfl_sync(0xffffffffu, myKey, __ffs(pending) - 1);
+    const unsigned left = r.state == kLeafPending ? unsigned(__popcll(r.leaves)) + 1u : 0u;
+    const int from = __ffs(__ballot_sync(0xffffffffu, left == __reduce_max_sync(0xffffffffu, left))) - 1;
+    const int key = __shfl_sync(0xffffffffu, myKey, from);
     const bool peer = r.state == kLeafPending && myKey == key;
     const unsigned peers = __ballot_sync(0xffffffffu, peer);
     // lanes are records: which of the group's can any peer's ray hit
