@@ -8,22 +8,25 @@
 // the reference's buffers, so there is no table-wide group cache; instead the
 // block keeps the groups its warps build (by the random-access grammar) in a
 // shared-memory table, and a warp that needs a group another warp of the block
-// has built reads it from there (neighbouring tiles reach the same groups: on
-// the bench poses a 16x16 block needs 6-9x fewer group builds than its warps
-// would alone).  Each ray still visits its leaves in the reference's order with
+// has built, or is building, reads it from there (neighbouring tiles reach the same
+// groups: on the bench poses a 16x16 block needs 6-9x fewer group builds than its
+// warps would alone).  Warps that came to a group while it was being built used to
+// build it too: six 1600x900 views, one call each, 5.69 ms, now 5.23 (16x16 blocks;
+// of 32x16 pixels 5.37, 8x16 6.65, fewer warps resident 6.07).  Each ray still visits its leaves in the reference's order with
 // the same running best, so Hit and Surface equal the reference's bit for bit.
 //
 // The reference's 64-row strips leave each launch a tail of partly idle SMs:
-// six 1600x900 views in 15 strips each trace in 24.4 ms, in one call per view
-// (rowCount = height, which the entry point accepts) in 14.3 ms.  A
+// six 1600x900 views in 15 strips each took 24.4 ms, in one call per view
+// (rowCount = height, which the entry point accepts) 14.3 ms, and in one call take
+// 5.23 now.  A
 // programmatic dependent launch of each strip was tried and measured no
 // faster: a dependent grid may be scheduled early, but its griddepcontrol.wait
 // returns only once the preceding grid has completed, and skipping that wait is
 // safe only when the preceding kernel is known to be another strip.
 #include <mutex>
 
-// (written out: six 3840x2160 views 23.7 ms in one call each, with one copy of each
-// division 24.7; blocks of eight warps here share more of their way through the code)
+// (written out: six 1600x900 views 5.23 ms, with one copy of each division 5.31; the
+// eight warps of a block share more of their way through the code)
 #define STRATUM_QUOTIENT WrittenOut
 #include "batch.cuh"
 #include "common_api.cuh"

@@ -312,51 +312,72 @@ struct WarpStage { StagedFeat feats[kEntryRecords]; };
 
 // Group records shared by the warps of one block, for a trace with no
 // table-wide group cache (the drop-in entry point).  Write-once for the
-// block's life: a warp that builds a group copies it into the next free entry
-// and then marks it ready; entries are never replaced, so a warp that finds a
-// ready entry reads the records in place.  Two warps that miss the same group
-// at once may both insert it (harmless).  At most 32 entries: one lane checks
-// each entry per lookup.
+// block's life: a warp that needs a group no entry names claims the next free
+// entry for it, builds the records there and marks it ready; a warp that needs a
+// group another warp is building waits for that, since the warps of a block set out
+// together and come to the same groups at the same time.  Entries are never
+// replaced, so the records are read in place.  At most 32 entries: one lane
+// checks each entry per lookup.
 #ifndef STRATUM_BLOCK_CACHE_ENTRIES
 #define STRATUM_BLOCK_CACHE_ENTRIES 32
 #endif
 constexpr int kBlockEntries = STRATUM_BLOCK_CACHE_ENTRIES;
 static_assert(kBlockEntries >= 1 && kBlockEntries <= 32, "one lane per block-cache entry");
+constexpr int kBlockWaits = 1024;  // of 64 ns or more; a build takes 2-5 us
 struct BlockCache {
   StagedFeat feats[kBlockEntries][kEntryRecords];
-  int key[kBlockEntries];
+  int key[kBlockEntries];  // -1: free
   int count[kBlockEntries];
   volatile int ready[kBlockEntries];
-  unsigned next;
 };
 // Every thread of the block calls this before any lookup (followed by a
 // block-wide barrier).
 SD void blockCacheInit(BlockCache& bc) {
-  for (int i = int(threadIdx.x); i < kBlockEntries; i += int(blockDim.x)) bc.ready[i] = 0;
-  if (threadIdx.x == 0) bc.next = 0u;
+  for (int i = int(threadIdx.x); i < kBlockEntries; i += int(blockDim.x)) {
+    bc.ready[i] = 0;
+    bc.key[i] = -1;
+  }
 }
-// The ready entry holding `key`, or -1.  Warp-collective.
-SD int blockCacheFind(const BlockCache& bc, int key) {
+// The entry for `key`, which this warp has to fill when `mine`; -1 when the table is
+// full.  Entries are claimed in order, so a warp that finds its key in none of them
+// and claims the first free one knows that no other has it; losing that entry to
+// another warp it looks again (at most once per entry).  Warp-collective.
+SD int blockCacheEntry(BlockCache& bc, int key, bool& mine) {
   const int lane = int(threadIdx.x & 31);
-  const int ready = lane < kBlockEntries ? bc.ready[lane] : 0;
-  // an entry's key and records were written before its ready flag: read them after it
+  mine = false;
+#pragma unroll 1
+  for (;;) {
+    const int held = lane < kBlockEntries ? reinterpret_cast<volatile int*>(bc.key)[lane] : -2;
+    const unsigned same = __ballot_sync(0xffffffffu, held == key), open = __ballot_sync(0xffffffffu, held == -1);
+    if (same) return __ffs(same) - 1;
+    if (!open) return -1;
+    const int e = __ffs(open) - 1;
+    int won = 0;
+    if (lane == 0) won = atomicCAS(&bc.key[e], -1, key) == -1;
+    if (__shfl_sync(0xffffffffu, won, 0)) {
+      mine = true;
+      return e;
+    }
+  }
+}
+// Whether the entry's records can be read, after a bounded wait.  Warp-collective.
+SD bool blockCacheReady(const BlockCache& bc, int e) {
+#pragma unroll 1
+  for (int i = 0; i < kBlockWaits; i++) {
+    if (__any_sync(0xffffffffu, bc.ready[e] != 0)) {
+      __threadfence_block();  // its records and count were written before its flag
+      return true;
+    }
+    __nanosleep(64);
+  }
+  return false;
+}
+// Mark an entry this warp has filled.  Warp-collective.
+SD void blockCachePublish(BlockCache& bc, int e, int count) {
+  if ((threadIdx.x & 31) == 0) bc.count[e] = count;
   __threadfence_block();
-  const bool hit = ready != 0 && reinterpret_cast<const volatile int*>(bc.key)[lane] == key;
-  const unsigned m = __ballot_sync(0xffffffffu, hit);
-  return m ? __ffs(m) - 1 : -1;
-}
-// Copy the group just staged in `ws` into a free entry, if any.  Warp-collective.
-SD void blockCachePut(BlockCache& bc, const WarpStage& ws, int key, int count) {
-  const int lane = int(threadIdx.x & 31);
-  unsigned e = 0u;
-  if (lane == 0) e = atomicAdd(&bc.next, 1u);
-  e = __shfl_sync(0xffffffffu, e, 0);
-  if (e >= unsigned(kBlockEntries)) return;
-  for (int k = lane; k < count; k += 32) bc.feats[e][k] = ws.feats[k];
-  if (lane == 0) { bc.key[e] = key; bc.count[e] = count; }
   __syncwarp();
-  __threadfence_block();
-  if (lane == 0) bc.ready[e] = 1;
+  if ((threadIdx.x & 31) == 0) bc.ready[e] = 1;
 }
 
 // Build one group's records by the grammar, one feature a lane, storing them
@@ -443,15 +464,17 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
                     StagedFeat& r0, StagedFeat& r1) {
   const int lane = int(threadIdx.x & 31);
   const int slot = key >> 6, g = key & 63;
-  const StagedFeat* feats = ws.feats;
+  StagedFeat* feats = ws.feats;
   uint32_t word = 0u;
-  int count, held = -1;
+  int count, entry = -1;
+  bool mine = true;
   if constexpr (kBlockCache) {
-    held = blockCacheFind(*bc, key);
-    if (held >= 0) {  // built earlier by a warp of this block
-      count = bc->count[held];
-      feats = bc->feats[held];
-    }
+    entry = blockCacheEntry(*bc, key, mine);
+    if (entry >= 0 && !mine) {
+      if (blockCacheReady(*bc, entry)) count = bc->count[entry];
+      else { entry = -1; mine = true; }
+    } else mine = true;
+    if (entry >= 0) feats = bc->feats[entry];
   } else if (cache.base) {
     const uint32_t row = lane < 9 ? __float_as_uint(__ldg(W + slot * kLotFloats + lane)) : 0u;
     word = __ldcg(cache.dir(slot, g));
@@ -473,11 +496,12 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
       }
     }
   }
-  if (held < 0) {
+  if (mine) {
     count = groupCount(loadLot(W, slot), g);
-    buildGroup(W, cache, key, count, word, ws.feats, nullptr);
+    buildGroup(W, cache, key, count, word, feats, nullptr);
     __syncwarp();
-    if constexpr (kBlockCache) blockCachePut(*bc, ws, key, count);
+    if constexpr (kBlockCache)
+      if (entry >= 0) blockCachePublish(*bc, entry, count);
   }
   r0 = feats[lane];
   r1 = feats[min(lane + 32, kEntryRecords - 1)];
