@@ -18,7 +18,7 @@
 // The reference's 64-row strips leave each launch a tail of partly idle SMs:
 // six 1600x900 views in 15 strips each took 24.4 ms, in one call per view
 // (rowCount = height, which the entry point accepts) 14.3 ms, and in one call take
-// 5.23 now.  A
+// 4.95 now.  A
 // programmatic dependent launch of each strip was tried and measured no
 // faster: a dependent grid may be scheduled early, but its griddepcontrol.wait
 // returns only once the preceding grid has completed, and skipping that wait is
@@ -130,11 +130,14 @@ extern "C" int stratum_tracePrimary(const float* World, const float* Nodes, cons
   });
   // Band rows: up to twice the blocks the device holds in quarter blocks, but at
   // most a sixth of a frame that fills the device by itself (a band row takes about
-  // two rows' time; a 64-row strip gets none).  One call, us, without / with: 320x180
-  // street 357 / 241, aerial 745 / 640; 640x360 street 535 / 360, canal 446 / 264;
-  // 1600x900 street 880 / 633, avenue 976 / 755, rooftop 860 / 950.
+  // two rows' time; a 64-row strip gets none), and none in one that fills it more than
+  // 14 times, whose other rows hide the slow tiles.  One call for each of six poses, sum
+  // in us, without / with: 320x180 2,045 / 1,507, 640x360 2,454 / 2,118, 1024x576 (7.8
+  // times) 3,380 / 3,167, 1283x721 (12.6) 4,125 / 4,099, 1600x900 (19) 4,948 / 5,238,
+  // 3840x2160 18,635 / 18,970.
   const int blocksX = (width + kDropInW - 1) / kDropInW, blockRows = (rows + kDropInH - 1) / kDropInH;
-  const int most = blocksX * blockRows <= resident[dev] ? blockRows : blockRows / 6;
+  const int blocks = blocksX * blockRows;
+  const int most = blocks <= resident[dev] ? blockRows : blocks <= 14 * resident[dev] ? blockRows / 6 : 0;
   const int want = (2 * resident[dev] - 1) / (4 * blocksX) + 1, bandRows = want < most ? want : most;
   tracePrimaryK<<<blocksX * (blockRows + 4 * bandRows), kDropInThreads, sizeof(DropInShared), asStream(stream)>>>(
       World, Nodes, static_cast<const uint32_t*>(Origin), C, Hit, Surface, width, height, rowStart, rowCount, blocksX,
