@@ -98,7 +98,7 @@ int stratum_schedulePages(const unsigned* Origin, const float* C, float* World, 
 /* commitPages = planBounds (Stratum.cu:186 role)                                */
 int stratum_commitPages(const unsigned* Queue, unsigned* Args, stratum_stream_t stream);
 /* buildBVH = buildGroupBounds + reduceGroupBounds x6 over the whole queue, as
- * one fused kernel (a block per lot; same bits).  Replaces the 8 x 7 indirect
+ * one fused kernel (eight lots a block; same bits).  Replaces the 8 x 7 indirect
  * dispatches of src/engine.js:71,74. */
 int stratum_buildBVH(const unsigned* Queue, const float* World, float* Nodes, stratum_stream_t stream);
 
@@ -244,7 +244,7 @@ int stratum_autotune(stratum_view* views, int n, void* scratch, unsigned long lo
  * memory to per-session tables), a foreign-language binding with no device
  * allocator, or a frame loop that must not allocate.  This variant keeps the
  * renderer's scratch (work-queue counters and per-view frame constants) in a
- * static device array of the library: about 6.9 KB, held by every GPU that
+ * static device array of the library: about 7.8 KB, held by every GPU that
  * loads the library until the process exits.  It allocates nothing and calls
  * no allocating routine.
  * Limits: at most STRATUM_NOALLOC_MAX_VIEWS views per call; more returns

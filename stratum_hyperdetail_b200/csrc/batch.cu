@@ -6,7 +6,7 @@
 //   stepViewsK      one thread per view: stepCamera
 //   clearViewsK,
 //   refreshViewsK   clearQueue + prepareLots of all views (grid: slots x views)
-//   buildViewsK     all views' queued lots, one 64-thread block per lot
+//   buildViewsK     all views' queued lots, eight to a block (hierarchy.cuh)
 //   prologueK       tile bases of every view under the chosen tile order, the
 //                   per-view frame constants (camera basis, sun, origin), the
 //                   resolve taps and the group caches' launch epochs, computed
@@ -176,10 +176,11 @@ SD void retire(uint32_t* next, uint32_t* done, int threads) {
   }
 }
 
-// STRATUM_TRACE_OCC / THREADS resident blocks (rounded down).  576 threads per SM
-// (112 registers): six-view 1600x900 frame 5.95 ms, aerial trace 1.90; 448 threads
-// 6.07 / 1.96, 512 6.06 / 1.95, 640 5.98 / 1.91, 768 (80 registers, spills) 5.97 / 1.87
-// but the small views' slowest tiles 5-10 % slower.
+// STRATUM_TRACE_OCC / THREADS resident blocks (rounded down).  At 576 threads per SM
+// the compiler takes 96 registers, which is ten 64-thread blocks: six-view 1600x900
+// trace 3.45 ms, aerial 1.54; 512 (128 registers) 3.73 / 1.69, 640 3.51 / 1.57.  768
+// (80 registers, spills) is equal over whole frames, but the slowest tiles, which bound
+// small views, take 5-10 % longer.
 #ifndef STRATUM_TRACE_OCC
 #define STRATUM_TRACE_OCC 576
 #endif
@@ -459,7 +460,7 @@ int render(stratum_view* V, int n, void* scratch, unsigned long long bytes, cons
 // The renderer's scratch (queue counters, resolve taps, per-view frame
 // constants) for callers that cannot give the library device memory, held in
 // one static device array.  Every GPU that loads the library holds this array
-// (about 6.9 KB) until the process exits.
+// (about 7.8 KB) until the process exits.
 constexpr int kNoAllocMaxViews = STRATUM_NOALLOC_MAX_VIEWS;
 constexpr size_t kNoAllocBytes = sizeof(BatchScratch) + size_t(kNoAllocMaxViews - 1) * sizeof(FrameConst);
 static __device__ __align__(256) unsigned char gNoAllocScratch[kNoAllocBytes];

@@ -6,7 +6,8 @@
 // Trace and shade cover the frame in one launch each.  The reference draws
 // 64-row strips (src/engine.js:76-77); a strip of 1,600 columns is 1.35 waves of
 // trace blocks and each launch ends in a tail of idle SMs, so six 1600x900
-// frames took 21.0 ms in strips and take 13.2 ms whole, with the same bits.
+// frames took 21.0 ms in strips and 13.2 ms whole (7.0 ms with the later kernels), with
+// the same bits.
 #include "../../include/stratum.h"
 
 extern "C" {

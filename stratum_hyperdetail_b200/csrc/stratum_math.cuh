@@ -60,8 +60,8 @@ HD float fract(float x) { return x - floorf(x); }
 // ---- divisions and square roots ----------------------------------------------
 // An IEEE division or square root takes 8-10 instructions and a branch where it is
 // written out.  The trace kernels run once through most of their code for each tile and
-// wait for instructions first of all, so they call one copy (OneCopy: 108 KB of
-// code to 90, six-view 1600x900 trace 4.62 -> 4.34 ms); shading loops over the same
+// wait for instructions first of all, so the batched one calls one copy (OneCopy: 108
+// KB of code to 90, six-view 1600x900 trace 4.62 -> 4.34 ms); shading loops over the same
 // code tile after tile and is faster with them written out (392 against 427 us for
 // the material pass).  Same results.
 struct WrittenOut {

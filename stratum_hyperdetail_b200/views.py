@@ -111,7 +111,7 @@ class View:
         for y in range(0, h, ROWS):
             call("stratum_shadePixels", ptr(self.World), ptr(self.Origin), ptr(self.C), ptr(self.Hit), ptr(self.Surface),
                  ptr(self.Linear), w, h, y, min(ROWS, h - y), s)
-            n += 1
+            n += 2  # material, then light
         call("stratum_resolveFrame", ptr(self.Linear), ptr(self.History), ptr(self.Pixels), ptr(self.C), ptr(self.Hit),
              ptr(self.Surface), w, h, s)
         return n + 1
