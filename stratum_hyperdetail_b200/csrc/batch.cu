@@ -462,7 +462,7 @@ int render(stratum_view* V, int n, void* scratch, unsigned long long bytes, cons
 // one static device array.  Every GPU that loads the library holds this array
 // (about 7.8 KB) until the process exits.
 constexpr int kNoAllocMaxViews = STRATUM_NOALLOC_MAX_VIEWS;
-constexpr size_t kNoAllocBytes = sizeof(BatchScratch) + size_t(kNoAllocMaxViews - 1) * sizeof(FrameConst);
+constexpr size_t kNoAllocBytes = batchScratchBytes(kNoAllocMaxViews);
 static __device__ __align__(256) unsigned char gNoAllocScratch[kNoAllocBytes];
 
 }  // namespace st

@@ -41,7 +41,7 @@ struct BatchScratch {
   ResolveTaps taps;
   ViewFrame view[1];  // n entries
 };
-inline size_t batchScratchBytes(int views) {
+constexpr size_t batchScratchBytes(int views) {
   return sizeof(BatchScratch) + size_t(views > 1 ? views - 1 : 0) * sizeof(ViewFrame);
 }
 
