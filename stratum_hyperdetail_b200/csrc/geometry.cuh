@@ -8,8 +8,8 @@
 
 namespace st {
 
-SD f3 intoFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(p.z, p.y, -p.x) : p; }
-SD f3 outOfFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(-p.z, p.y, p.x) : p; }
+HD f3 intoFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(p.z, p.y, -p.x) : p; }
+HD f3 outOfFeature(f3 p, int turn) { return (turn % 2 == 1) ? mk(-p.z, p.y, p.x) : p; }
 
 SD f3 leafNormal(int x, int y, int z, int seed) {  // geometry.cu:6-8
   return Quotient::unit(mk(hash2(x + y * 19, z, seed) - 0.5f, 0.25f + hash2(x - y, z + 91, seed) * 0.7f,
@@ -59,7 +59,7 @@ static __device__ __noinline__ float foliageHit(f3 ro, f3 rd, f3 centre, f3 radi
 
 // Four fixed-point steps of the ray against the mortar height field
 // (geometry.cu:82-89).  Called only for tall stone/brick boxes.
-static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f3 d, float t, float cone) {
+static __host__ __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f3 d, float t, float cone) {
   const f3 h = f.h;
   // Beyond freqWeight's cut-off (t * cone >= 0.0275: 23 m at 900 rows) the relief
   // is multiplied by exactly 0 and every step leaves t where it is; without this
@@ -90,11 +90,11 @@ static __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f
 // Nearest positive hit of one feature, kFar if none (geometry.cu:33-91), in two
 // parts: the slab test every feature starts with (`p`, `d` are the ray in the
 // feature's frame and `inv` = invDir<Quotient>(d)), and the rest.
-SD Span featureSlab(const Feat& f, f3 p, f3 inv) {
+HD Span featureSlab(const Feat& f, f3 p, f3 inv) {
   const f3 h = f.h;
   return (f.shape == 3 || f.shape == 4) ? slabInv(p, inv, mk(-h.x, 0.0f, -h.z), h) : slabInv(p, inv, h * -1.0f, h);
 }
-SD bool featureSlabMiss(const Feat& f, Span range) { return f.shape < 0 || range.hi < fmaxf(0.001f, range.lo); }
+HD bool featureSlabMiss(const Feat& f, Span range) { return f.shape < 0 || range.hi < fmaxf(0.001f, range.lo); }
 // What follows a passed slab test of that range.
 SD float featureInSlab(const Feat& f, f3 ro, f3 rd, f3 p, f3 d, Span range, float cone) {
   const int shape = f.shape;

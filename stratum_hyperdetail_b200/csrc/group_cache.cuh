@@ -42,12 +42,12 @@ struct alignas(16) StagedFeat {
   int packed;  // shape + 1 | material << 8 | turn << 16
   float seed;
 };
-SD void stage(StagedFeat& s, const Feat& f) {
+HD void stage(StagedFeat& s, const Feat& f) {
   s.px = f.p.x; s.py = f.p.y; s.pz = f.p.z; s.hx = f.h.x; s.hy = f.h.y; s.hz = f.h.z;
   s.packed = (f.shape + 1) | (f.material << 8) | (f.turn << 16);
   s.seed = f.seed;
 }
-SD Feat unstage(const StagedFeat& s) {
+HD Feat unstage(const StagedFeat& s) {
   return Feat{mk(s.px, s.py, s.pz), mk(s.hx, s.hy, s.hz), (s.packed & 255) - 1, (s.packed >> 8) & 255,
               (s.packed >> 16) & 255, s.seed};
 }

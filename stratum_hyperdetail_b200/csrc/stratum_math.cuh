@@ -69,13 +69,13 @@ struct WrittenOut {
   static HD float root(float a) { return sqrtf(a); }
   static HD f3 unit(f3 a) { return st::unit(a); }
 };
-static __device__ __noinline__ float divideOnce(float a, float b) { return a / b; }
-static __device__ __noinline__ float rootOnce(float a) { return sqrtf(a); }
-static __device__ __noinline__ f3 unitOnce(f3 a) { return unit(a); }
+static __host__ __device__ __noinline__ float divideOnce(float a, float b) { return a / b; }
+static __host__ __device__ __noinline__ float rootOnce(float a) { return sqrtf(a); }
+static __host__ __device__ __noinline__ f3 unitOnce(f3 a) { return unit(a); }
 struct OneCopy {
-  static SD float div(float a, float b) { return divideOnce(a, b); }
-  static SD float root(float a) { return rootOnce(a); }
-  static SD f3 unit(f3 a) { return unitOnce(a); }
+  static HD float div(float a, float b) { return divideOnce(a, b); }
+  static HD float root(float a) { return rootOnce(a); }
+  static HD f3 unit(f3 a) { return unitOnce(a); }
 };
 // How a file's kernels divide in the code they share (a file defines
 // STRATUM_QUOTIENT before its includes to choose otherwise).

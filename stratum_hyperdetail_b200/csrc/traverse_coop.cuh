@@ -58,12 +58,11 @@ static __device__ __noinline__ Feat featureAtOOL(LotDesc L, int g, int i) { retu
 
 // A box (in the lot frame) that contains every distance a feature can return: a
 // lane tests a feature only when its ray enters that box nearer than its
-// current best, so a skipped feature could only have been rejected and
-// results are unchanged.  That holds for the features whose computed distance
-// is a slab entry of their own box or follows from it: plain boxes and prisms
-// (the slab entry, or a roof plane behind it), masonry boxes (relief moves the
-// hit at most 0.0025 m toward the ray per unit of the face normal, inside the
-// 0.025 m pad) and foliage envelopes (leaf discs reach at most one 0.18 m grid
+// current best (and kReliefReach beyond it), so a skipped feature could only have
+// been rejected and results are unchanged.  That holds for the features whose
+// computed distance is a slab entry of their own box or follows from it: plain
+// boxes and prisms (the slab entry, or a roof plane behind it), masonry boxes (see
+// kReliefReach) and foliage envelopes (leaf discs reach at most one 0.18 m grid
 // cell, 0.31 m diagonal, beyond the envelope's box: 0.35 m pad).  Ellipsoids,
 // cylinders and arches/rings solve a quadratic whose float result can land
 // well outside the box at long range (cancellation; 0.17 m at 1.4 km was
@@ -80,7 +79,13 @@ static __device__ __noinline__ Feat featureAtOOL(LotDesc L, int g, int i) { retu
 constexpr int kRun = STRATUM_COOP_RUN;
 static_assert(kRun * kEntryBoxes >= kEntryRecords, "a group cache entry holds every chunk box of a group");
 struct ChunkBox { float lo[3], hi[3]; };
-SD void hitBox(const Feat& f, f3& lo, f3& hi) {
+// How far the entry of a masonry box's padded box may lie behind its hit.  Relief moves
+// the hit up to 0.0025 m off the face, and faces of a slant down to 0.08 have it: 0.03125 m
+// along the ray.  The entry of the box by another axis, which the ray may cross at
+// right angles, lies no more than the pad's 0.025 m before the unmoved hit.  So 0.00625 m,
+// and the rounding at 2 km.
+constexpr float kReliefReach = 0.01f;
+HD void hitBox(const Feat& f, f3& lo, f3& hi) {
   const bool foliage = f.shape == 1 && f.material == 7;
   f3 ext = f.h;
   if (f.turn % 2 == 1) ext = mk(f.h.z, f.h.y, f.h.x);
@@ -111,12 +116,12 @@ struct Packet { f3 ro, lo, hi; float best; };
 // packet they lie between the extremes of the four products of the box's two
 // planes with the interval's two ends; a record is out when the latest of the
 // axes' earliest entries is past the earliest of their latest exits, or past
-// every ray's best.  The latter holds for boxes (masonry relief included, inside the
-// pad) and prisms only: quadrics and foliage are bounded by the box test alone.
+// every ray's best by more than kReliefReach.  The latter holds for boxes (masonry
+// relief included) and prisms only: quadrics and foliage are bounded by the box test alone.
 // The 0.025 m pad covers every rounding of this test and of the exact one: at
 // |ro| <= 2,100 m (a visited lot is at most 2,000 m along a ray) they sum to
 // less than 0.001 m.
-SD bool packetEnters(const Packet& k, f3 lo, f3 hi, float& in) {
+HD bool packetEnters(const Packet& k, f3 lo, f3 hi, float& in) {
   const float ax = lo.x - k.ro.x, bx = hi.x - k.ro.x, ay = lo.y - k.ro.y, by = hi.y - k.ro.y;
   const float az = lo.z - k.ro.z, bz = hi.z - k.ro.z;
   const float x0 = ax * k.lo.x, x1 = ax * k.hi.x, x2 = bx * k.lo.x, x3 = bx * k.hi.x;
@@ -129,18 +134,25 @@ SD bool packetEnters(const Packet& k, f3 lo, f3 hi, float& in) {
   return in <= out && out >= 0.001f;
 }
 // Whether some ray may enter this node's box nearer than its own best.
-SD bool packetMayEnter(float4 a, float4 b, const Packet& k) {
+HD bool packetMayEnter(float4 a, float4 b, const Packet& k) {
   const float pad = 0.01f;
   float in;
   return packetEnters(k, mk(a.x - pad, a.y - pad, a.z - pad), mk(b.x + pad, b.y + pad, b.z + pad), in) && in <= k.best;
 }
-SD bool packetMayHit(const StagedFeat& s, const Packet& k) {
+HD bool packetMayHit(const StagedFeat& s, const Packet& k) {
   const int shape = (s.packed & 255) - 1;
   const bool odd = (s.packed >> 16) & 1, base = shape == 3 || shape == 4;  // these stand on p.y
   const float hx = (odd ? s.hz : s.hx) + 0.025f, hz = (odd ? s.hx : s.hz) + 0.025f, hy = s.hy + 0.025f;
   float in;
   return packetEnters(k, mk(s.px - hx, base ? s.py - 0.025f : s.py - hy, s.pz - hz), mk(s.px + hx, s.py + hy, s.pz + hz), in) &&
-         (in <= k.best || !(shape == 0 || shape == 3));
+         (in <= k.best + kReliefReach || !(shape == 0 || shape == 3));
+}
+// Whether a ray may hit this record, neither a plain box nor a prism, nearer than `best`.
+HD bool mayWin(const Feat& f, f3 ro, f3 inv, float best) {
+  f3 lo, hi;
+  hitBox(f, lo, hi);
+  const Span r = slabInv(ro, inv, lo, hi);
+  return !(r.hi < fmaxf(0.001f, r.lo) || r.lo > best + kReliefReach);
 }
 
 enum LaneState : int { kEnterLot = 0, kLotPending = 1, kLeafPending = 2, kDone = 3, kNextLeaf = 4 };
@@ -610,11 +622,8 @@ SD TraceResult traceWarp(const float* __restrict__ W, const float4* __restrict__
           const f3 d = odd ? mk(r.ld.z, r.ld.y, -r.ld.x) : r.ld;
           if (f.shape == 3) {  // its distance is never before the slab's entry
             if (rg.lo > r.best || prismMiss(f, p, d, rg)) continue;
-          } else {
-            f3 lo, hi;
-            hitBox(f, lo, hi);
-            const Span cr = slabInv(r.lr, r.inv0, lo, hi);
-            if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > r.best) continue;  // it cannot win
+          } else if (!mayWin(f, r.lr, r.inv0, r.best)) {
+            continue;
           }
           th = featureInSlabOOL(f, r.lr, r.ld, p, d, rg, r.cone);
         }

@@ -51,7 +51,7 @@ SD void poolTest(PoolShared<P>& sh, int j, const PoolStage& ws, int count, int g
   for (int c = 0; c * kRun < count; c++) {
     const ChunkBox b = ws.boxes[c];
     const Span cr = slabInv(lr, inv0, mk(b.lo[0], b.lo[1], b.lo[2]), mk(b.hi[0], b.hi[1], b.hi[2]));
-    if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > best) continue;  // no feature of the run can win
+    if (cr.hi < fmaxf(0.001f, cr.lo) || cr.lo > best + kReliefReach) continue;  // no feature of the run can win
     const int kEnd = min(count, (c + 1) * kRun);
 #pragma unroll 1
     for (int k = c * kRun; k < kEnd; k++) {
