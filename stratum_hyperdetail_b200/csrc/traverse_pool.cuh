@@ -29,13 +29,19 @@ struct PoolShared {
   PoolStage stage[P];
   float lr[3][P * 32], ld[3][P * 32], inv[3][P * 32];
   float best[P * 32], cone[P * 32];
-  int key[P * 32];  // pending head (view << 20 | slot << 6 | group), or -1
-  int fid[P * 32];  // winner (group * 64 + index) after a serve that improved best
+  unsigned long long key[P * 32];  // pending head (poolKey), or kPoolIdle
+  int fid[P * 32];                 // winner (group * 64 + index) after a serve that improved best
 };
 
-SD int poolKey(int view, int slot, int group) { return (view << 20) | (slot << 6) | group; }
+// A head of any view a launch takes (65,535: 36 bits).
+constexpr unsigned long long kPoolIdle = ~0ull;
+HD unsigned long long poolKey(int view, int slot, int group) {
+  return (unsigned long long)view << 20 | unsigned(slot << 6 | group);
+}
+HD int poolView(unsigned long long key) { return int(key >> 20); }
+HD int poolGroupKey(unsigned long long key) { return int(key & 0xFFFFFu); }  // slot << 6 | group
 template <int P>
-SD int poolWarpOf(int key) { return int((unsigned(key) * 2654435761u) >> 16) % P; }
+SD int poolWarpOf(unsigned long long key) { return int((unsigned(key) * 2654435761u) >> 16) % P; }
 
 // One ray of the block against the group staged in `ws` (the record loop of
 // traceWarp, on the ray's state in shared memory).
@@ -80,20 +86,20 @@ SD void poolTest(PoolShared<P>& sh, int j, const PoolStage& ws, int count, int g
 template <int P>
 SD void poolServe(PoolShared<P>& sh, const stratum_view* __restrict__ V) {
   const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-  int kk[P];
+  unsigned long long kk[P];
   unsigned mine[P];
 #pragma unroll
   for (int p = 0; p < P; p++) {
     kk[p] = sh.key[p * 32 + lane];
-    mine[p] = __ballot_sync(0xffffffffu, kk[p] >= 0 && poolWarpOf<P>(kk[p]) == warp);
+    mine[p] = __ballot_sync(0xffffffffu, kk[p] != kPoolIdle && poolWarpOf<P>(kk[p]) == warp);
   }
 #pragma unroll 1
   for (;;) {
-    int key = -1;
+    unsigned long long key = kPoolIdle;
 #pragma unroll
     for (int p = 0; p < P; p++)
-      if (key < 0 && mine[p]) key = __shfl_sync(0xffffffffu, kk[p], __ffs(mine[p]) - 1);
-    if (key < 0) break;
+      if (key == kPoolIdle && mine[p]) key = __shfl_sync(0xffffffffu, kk[p], __ffs(mine[p]) - 1);
+    if (key == kPoolIdle) break;
     unsigned wait[P];
     int total = 0;
 #pragma unroll
@@ -102,9 +108,9 @@ SD void poolServe(PoolShared<P>& sh, const stratum_view* __restrict__ V) {
       mine[p] &= ~wait[p];
       total += __popc(wait[p]);
     }
-    const int v = key >> 20, slot = (key >> 6) & (kLots - 1), g = key & 63;
+    const int v = poolView(key), gk = poolGroupKey(key), g = gk & 63;
     PoolStage& ws = sh.stage[warp];
-    const int count = stageGroup(V[v].World, groupCache(V[v].Groups), (slot << 6) | g, ws.feats, ws.boxes);
+    const int count = stageGroup(V[v].World, groupCache(V[v].Groups), gk, ws.feats, ws.boxes);
     __syncwarp();
     // the waiting rays, compacted: lane i takes the i-th of each 32
 #pragma unroll 1
@@ -142,7 +148,7 @@ SD TraceResult tracePooled(PoolShared<P>& sh, const stratum_view* __restrict__ V
       sh.best[tid] = r.best;
       sh.cone[tid] = r.cone;
     }
-    sh.key[tid] = pend ? poolKey(view, r.slot, r.pend) : -1;
+    sh.key[tid] = pend ? poolKey(view, r.slot, r.pend) : kPoolIdle;
     if (!__syncthreads_or(pend)) break;  // every ray of the block is done
 #pragma unroll 1
     for (;;) {
@@ -157,7 +163,7 @@ SD TraceResult tracePooled(PoolShared<P>& sh, const stratum_view* __restrict__ V
         }
         nextLeaf(r, N);
         pend = r.state == kLeafPending;
-        sh.key[tid] = pend ? poolKey(view, r.slot, r.pend) : -1;
+        sh.key[tid] = pend ? poolKey(view, r.slot, r.pend) : kPoolIdle;
       }
       if (!__syncthreads_or(pend)) break;
     }

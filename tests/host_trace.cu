@@ -1,7 +1,8 @@
-// Test infrastructure: the trace's record culls compiled for the HOST, against the
-// distance of the same record, for a CPU comparison.
+// Test infrastructure: what the traces decide by, compiled for the HOST: the record
+// culls against the distance of the same record, and the heads of the block-pooled form.
 #define STRATUM_QUOTIENT WrittenOut
-#include "traverse_coop.cuh"
+#include "common_api.cuh"
+#include "traverse_pool.cuh"
 
 using namespace st;
 
@@ -30,4 +31,16 @@ extern "C" void ht_culls(const float* boxes, const float* rays, int n, float con
     stage(s, f);
     kept[i] = (packetMayHit(s, Packet{ro, inv, inv, best}) ? 1 : 0) | (mayWin(f, ro, inv, best) ? 2 : 0);
   }
+}
+
+// The block-pooled trace's heads of n (view, slot, group): whether each is told from an
+// idle lane and read back as it was.
+extern "C" int ht_heads(const int* heads, int n) {
+  int good = 0;
+  for (int i = 0; i < n; i++) {
+    const int v = heads[3 * i], slot = heads[3 * i + 1], g = heads[3 * i + 2];
+    const unsigned long long k = poolKey(v, slot, g);
+    good += k != kPoolIdle && poolView(k) == v && poolGroupKey(k) == (slot << 6 | g);
+  }
+  return good;
 }

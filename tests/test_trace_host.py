@@ -1,5 +1,5 @@
-"""The trace's record culls on the CPU: a record that a ray hits nearer than its best
-passes them.
+"""What the traces decide by, on the CPU.  A record that a ray hits nearer than its best
+passes the culls, and a pooled head names its view.
 
 Relief moves a tall stone or brick box's hit toward the camera by up to 0.0025 m
 per unit of the face's slant, which goes down to 0.08: 0.031 m along a grazing ray,
@@ -31,9 +31,10 @@ def ht(tmp_path_factory):
     out = tmp_path_factory.mktemp("ht") / "libht.so"
     subprocess.run([nvcc, "-x", "cu", "-std=c++17", "-O2", "-shared", "--fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler",
                     "-ffp-contract=off", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(CSRC), "-I", str(GEN),
-                    str(ROOT / "tests" / "host_trace.cu"), "-o", str(out)], check=True)
+                    "-I", str(ROOT / "include"), str(ROOT / "tests" / "host_trace.cu"), "-o", str(out)], check=True)
     lib = ct.CDLL(str(out))
     lib.ht_culls.argtypes = [f32p, f32p, ct.c_int, ct.c_float, f32p, i32p]
+    lib.ht_heads.argtypes = [i32p, ct.c_int]
     return lib
 
 
@@ -63,3 +64,10 @@ def test_grazed_relief_passes_the_culls(ht, steep, along, far):
     for bit, name in ((1, "packet"), (2, "ray")):
         lost = hits & ((kept & bit) == 0)
         assert not lost.any(), (name, int(lost.sum()), boxes[lost][0], rays[lost][0], t[lost][0])
+
+
+def test_pooled_heads_of_every_view(ht):
+    """65,535 views is the most that a batched call takes."""
+    heads = np.array([(v, s, g) for v in (0, 1, 2047, 2048, 4095, 4096, 32768, 65534) for s in (0, 1, 8191, 16383)
+                      for g in (0, 31, 63)], np.int32)
+    assert ht.ht_heads(np.ascontiguousarray(heads), len(heads)) == len(heads)
