@@ -124,13 +124,23 @@ SD uint32_t acquireWord(const uint32_t* p) {
   return v;
 }
 
+// Directory words change while a launch runs, and lanes that load the same word for
+// themselves need not see the same value of it.  Whatever a warp decides by a word is
+// therefore decided by lane 0 for all of it, so that its lanes reach the same
+// warp-wide steps.
+
+// The entry lane 0's directory word names if it was filled by an earlier launch, else -1.
+// Warp-collective.
+SD int warpEntry(const GroupCache& c, uint32_t word) { return __shfl_sync(0xffffffffu, usableEntry(c, word), 0); }
+
 // Warp-collective: claim a fresh entry for (slot, group), or -1 when another
 // warp is filling it, filled it in this launch, or the store is full.  `old`
-// is the directory word the caller read.  A claimed entry must be published.
+// is the directory word the caller read (lane 0's counts).  A claimed entry must be
+// published.
 SD int cacheClaim(const GroupCache& c, int slot, int group, uint32_t old) {
-  if (c.capacity() == 0u || old == kCacheBusy || (old != 0u && (old >> 24) == c.epoch())) return -1;
+  if (c.capacity() == 0u) return -1;  // set before the launch: the same for every lane
   int e = -1;
-  if ((threadIdx.x & 31) == 0) {
+  if ((threadIdx.x & 31) == 0 && old != kCacheBusy && (old == 0u || (old >> 24) != c.epoch())) {
     uint32_t* dp = c.dir(slot, group);
     if (__ldcg(&c.hdr()->next) < c.capacity() && atomicCAS(dp, old, kCacheBusy) == old) {
       const uint32_t i = atomicAdd(&c.hdr()->next, 1u);
@@ -155,11 +165,14 @@ SD void cachePublish(const GroupCache& c, const float* W, int slot, int group, i
 }
 
 // The entry a directory word names if this launch filled it and it can be read now,
-// else -1; `word` is read again.
+// else -1; `word` is read again.  The other lanes read the entry after the barrier, and so
+// after lane 0's acquire.  Warp-collective.
 SD int filledNow(const GroupCache& c, uint32_t& word, int slot, int group) {
-  if (freshEntry(c, word) < 0) return -1;
+  if (__shfl_sync(0xffffffffu, freshEntry(c, word), 0) < 0) return -1;
   word = acquireWord(c.dir(slot, group));
-  return freshEntry(c, word);
+  const int e = __shfl_sync(0xffffffffu, freshEntry(c, word), 0);
+  __syncwarp();
+  return e;
 }
 
 // Record i of an entry filled by an earlier launch (read-only here), and by this one.

@@ -442,7 +442,7 @@ SD int stageGroup(const float* __restrict__ W, const GroupCache& cache, int key,
   // kept only if every tag word matches the slot's current descriptor (else a miss)
   const uint32_t word = cache.base ? __ldcg(cache.dir(slot, g)) : 0u;
   const int count = groupCount(loadLot(W, slot), g);
-  const int e = cache.base ? usableEntry(cache, word) : -1;
+  const int e = cache.base ? warpEntry(cache, word) : -1;
   if (e >= 0) {
     bool same = true;
     if (lane < kEntryTagWords)
@@ -490,7 +490,7 @@ SD int groupRecords(const float* __restrict__ W, const GroupCache& cache, BlockC
   } else if (cache.base) {
     const uint32_t row = lane < 9 ? __float_as_uint(__ldg(W + slot * kLotFloats + lane)) : 0u;
     word = __ldcg(cache.dir(slot, g));
-    const int e = usableEntry(cache, word);
+    const int e = warpEntry(cache, word);
     if (e >= 0) {
       const uint32_t tag = lane < kEntryTagWords ? __ldg(entryTag(cache, uint32_t(e)) + lane) : 0u;
       r0 = cacheRecord(cache, e, lane);
