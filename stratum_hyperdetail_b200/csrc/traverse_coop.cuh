@@ -378,6 +378,7 @@ SD bool blockCacheReady(const BlockCache& bc, int e) {
   for (int i = 0; i < kBlockWaits; i++) {
     if (__any_sync(0xffffffffu, bc.ready[e] != 0)) {
       __threadfence_block();  // its records and count were written before its flag
+      __syncwarp();           // which some lanes may not have seen yet
       return true;
     }
     __nanosleep(64);
