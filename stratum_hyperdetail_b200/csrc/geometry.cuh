@@ -61,12 +61,13 @@ static __device__ __noinline__ float foliageHit(f3 ro, f3 rd, f3 centre, f3 radi
 // (geometry.cu:82-89).  Called only for tall stone/brick boxes.
 static __host__ __device__ __noinline__ float masonryRelief(Feat f, f3 ro, f3 rd, f3 p, f3 d, float t, float cone) {
   const f3 h = f.h;
+  f3 hp = p + d * t;
   // Beyond freqWeight's cut-off (t * cone >= 0.0275: 23 m at 900 rows) the relief
   // is multiplied by exactly 0 and every step leaves t where it is; without this
   // return the four height-field steps of far walls took 13 % of the six-view
-  // 1600x900 trace (6.80 -> 5.91 ms, aerial pose 2.89 -> 2.39 ms).
-  if (freqWeight<Quotient>(t * cone, 40.0f) == 0.0f) return t;
-  f3 hp = p + d * t;
+  // 1600x900 trace (6.80 -> 5.91 ms, aerial pose 2.89 -> 2.39 ms).  (Noise at a point that
+  // is not finite is no number, and 0 times it is none either: such a ray misses.)
+  if (fabsf(hp.x) + fabsf(hp.y) + fabsf(hp.z) < 1e30f && freqWeight<Quotient>(t * cone, 40.0f) == 0.0f) return t;
   float ex = fabsf(fabsf(hp.x) - h.x), ez = fabsf(fabsf(hp.z) - h.z);
   if (fabsf(fabsf(hp.y) - h.y) > 0.01f) {
     f3 n = ex < ez ? mk(hp.x < 0.0f ? -1.0f : 1.0f, 0.0f, 0.0f) : mk(0.0f, 0.0f, hp.z < 0.0f ? -1.0f : 1.0f);

@@ -34,6 +34,7 @@ def ht(tmp_path_factory):
                     "-I", str(ROOT / "include"), str(ROOT / "tests" / "host_trace.cu"), "-o", str(out)], check=True)
     lib = ct.CDLL(str(out))
     lib.ht_culls.argtypes = [f32p, f32p, ct.c_int, ct.c_float, f32p, i32p]
+    lib.ht_relief.argtypes = [f32p, f32p, f32p, f32p, ct.c_int, f32p, f32p]
     lib.ht_heads.argtypes = [i32p, ct.c_int]
     return lib
 
@@ -71,3 +72,26 @@ def test_pooled_heads_of_every_view(ht):
     heads = np.array([(v, s, g) for v in (0, 1, 2047, 2048, 4095, 4096, 32768, 65534) for s in (0, 1, 8191, 16383)
                       for g in (0, 31, 63)], np.int32)
     assert ht.ht_heads(np.ascontiguousarray(heads), len(heads)) == len(heads)
+
+
+@pytest.mark.parametrize("value", [None, float("nan"), float("inf"), -float("inf"), 1e38])
+def test_relief_leaves_out_only_steps_that_come_to_nothing(ht, value):
+    """Footprints on both sides of the cut-off, and rays that are not finite: a distance
+    that is no number (a miss) stays none."""
+    n = 100000
+    rng = np.random.default_rng(11)
+    half = rng.uniform(1.05, 9, (n, 3))
+    boxes = np.concatenate([rng.uniform(-12, 12, (n, 3)), half, rng.integers(0, 2, (n, 1))], 1).astype(np.float32)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    start = rng.uniform(0.1, 300.0, n)
+    face = boxes[:, :3] + np.where(rng.random((n, 3)) < 0.5, -1, 1) * half * rng.choice([1.0, 0.3], (n, 3))
+    rays = np.concatenate([face - d * start[:, None], d], 1)
+    if value is not None:
+        rays[np.arange(n), rng.integers(0, 6, n)] = value
+    rays, start = rays.astype(np.float32), start.astype(np.float32)
+    cone = np.where(rng.random(n) < 0.5, 0.0275 / start * rng.uniform(0.5, 1.5, n), 0.01).astype(np.float32)
+    t, whole = np.zeros(n, np.float32), np.zeros(n, np.float32)
+    ht.ht_relief(boxes, rays, start, cone, n, t, whole)
+    assert np.array_equal(t, whole, equal_nan=True)
+    assert (whole != start).sum() > 1000
