@@ -15,7 +15,8 @@ namespace st {
 //
 // What bounds shading is instruction issue, then instruction fetch.  Work whose
 // result is certain is left out below, always to the same bits: noise with a
-// weight of exactly 0, the sun's powers where they are 0, a lot's inverse
+// weight of exactly 0 (at a finite point: elsewhere it is no number, and stays
+// none), the sun's powers where they are 0, a lot's inverse
 // directions by permuting the light's, masses below the point, and resolve taps
 // that cannot occlude.  Six 1600x900 views: material 455 -> 392 us, light 875 -> 736,
 // resolve 712 -> 611.
@@ -61,11 +62,14 @@ SD f3 mineralCell(float u, float v, int seed) {
     }
   return mk(sqrtf(nearest), value, sqrtf(second) - sqrtf(nearest));
 }
+// Whether noise at these coordinates, times any frequency used here, is a number.
+SD bool noiseIsFinite(float u, float v) { return fabsf(u) < 1e30f && fabsf(v) < 1e30f; }
 SD float microRelief(float u, float v, float fp) {
   const float mid = freqWeight(fp, 277.0f), high = freqWeight(fp, 911.0f);
   float value = (noise2D(u * 83.0f, v * 83.0f) - 0.5f) * 0.0016f * freqWeight(fp, 83.0f);
-  if (mid > 0.0f) value += (noise2D(u * 277.0f + 8.7f, v * 277.0f) - 0.5f) * 0.00048f * mid;
-  if (high > 0.0f) value += (noise2D(u * 911.0f, v * 911.0f - 13.9f) - 0.5f) * 0.00013f * high;
+  const bool all = !noiseIsFinite(u, v);
+  if (mid > 0.0f || all) value += (noise2D(u * 277.0f + 8.7f, v * 277.0f) - 0.5f) * 0.00048f * mid;
+  if (high > 0.0f || all) value += (noise2D(u * 911.0f, v * 911.0f - 13.9f) - 0.5f) * 0.00013f * high;
   return value;
 }
 // Terms whose frequency weight is exactly 0 at this footprint (1.1 / frequency and
@@ -74,6 +78,7 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
   float u, v;
   masonryUV(p, n, u, v);
   float fine = freqWeight(fp, 34.0f);
+  const bool finite = noiseIsFinite(u, v);
   f3 c = foundation;
   if (mat == 0 || mat == 1) {  // brick / stone with joints, pores, minerals, cracks, moss
     float bw = mat == 1 ? 0.46f : 0.92f, bh = mat == 1 ? 0.215f : 0.46f;
@@ -100,7 +105,7 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
       c = c * (1.0f + powder * (joint > 0.5f ? 0.50f : 0.24f));
     }
     const float cracks = freqWeight(fp, 15.0f);
-    if (cracks > 0.0f) {
+    if (cracks > 0.0f || !finite) {
       float crack = fabsf(sinf(u * 8.4f + fbm2D(u * 2.4f, v * 2.4f) * 5.0f + v * 1.3f));
       float fracture = (1.0f - smooth(0.012f, 0.042f + fp * 4.0f, crack)) * smooth(0.48f, 0.72f, noise2D(u * 1.4f, v * 1.4f));
       c = c * (1.0f - fracture * 0.45f * cracks);
@@ -112,7 +117,7 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
     float tile = fract(u * 3.7f), row = fract(v * 4.4f);
     float seam = (1.0f - smooth(0.01f, 0.07f, tile)) + (1.0f - smooth(0.02f, 0.11f, row));
     const float mottle = freqWeight(fp, 7.2f);
-    c = c * (0.78f + 0.26f * (mottle > 0.0f ? lerp(0.5f, noise2D(u * 7.2f, v * 7.2f), mottle) : 0.5f) -
+    c = c * (0.78f + 0.26f * (mottle > 0.0f || !finite ? lerp(0.5f, noise2D(u * 7.2f, v * 7.2f), mottle) : 0.5f) -
              sat(seam) * 0.25f * freqWeight(fp, 4.4f));
   } else if (mat == 3) {  // copper patina
     float patina = smooth(0.28f, 0.64f, fbm2D(u * 2.1f, v * 2.1f));
@@ -122,7 +127,7 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
   } else if (mat == 4) c = mk(0.045f, 0.084f, 0.093f);
   else if (mat == 5) {
     c = mk(0.12f, 0.07f, 0.039f);
-    if (fine > 0.0f) c = c * (1.0f + sinf(u * 49.0f + fbm2D(u * 2.0f, v * 0.5f) * 8.0f) * 0.12f * fine);
+    if (fine > 0.0f || !finite) c = c * (1.0f + sinf(u * 49.0f + fbm2D(u * 2.0f, v * 0.5f) * 8.0f) * 0.12f * fine);
   } else if (mat == 6) c = mk(0.075f, 0.091f, 0.087f) * (0.8f + noise2D(u * 30.0f, v * 30.0f) * 0.3f);
   else if (mat == 7) {
     float leaves = fbm2D(p.x * 8.0f + p.y * 6.0f, p.z * 8.0f);
@@ -131,7 +136,7 @@ static __device__ __noinline__ f3 surfaceColor(f3 p, f3 n, int mat, float seed, 
   else if (mat == 9) c = mk(0.035f, 0.115f, 0.12f);
   else if (mat == 10) {
     const float gravel = freqWeight(fp, 45.0f);
-    float grit = gravel > 0.0f ? lerp(0.5f, fbm2D(u * 45.0f, v * 45.0f), gravel) : 0.5f;
+    float grit = gravel > 0.0f || !finite ? lerp(0.5f, fbm2D(u * 45.0f, v * 45.0f), gravel) : 0.5f;
     c = mk(0.16f, 0.17f, 0.16f) * (0.72f + grit * 0.4f);
   } else if (mat == 11) {
     int row = int(floorf(v / 0.45f));
@@ -296,7 +301,7 @@ SD f3 pixelLight(const float* __restrict__ W, const FrameConst& F, const Surface
   if ((mat == 0 || mat == 1) && fabsf(qn.y) < 0.5f) {  // mortar relief normal by central differences
     const float fade = freqWeight(sfp, 5.0f);
     float eps = fmaxf(0.002f, sfp * 0.6f), du = 0.0f, dv = 0.0f;
-    if (fade > 0.0f) {
+    if (fade > 0.0f || !noiseIsFinite(u, v)) {
       du = (masonryHeightD(u + eps, v, mat) - masonryHeightD(u - eps, v, mat)) / (2.0f * eps);
       dv = (masonryHeightD(u, v + eps, mat) - masonryHeightD(u, v - eps, mat)) / (2.0f * eps);
       if (sfp < 0.005f) {
