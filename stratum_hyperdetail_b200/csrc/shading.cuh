@@ -196,7 +196,8 @@ SD float ambientVisibility(const float* __restrict__ W, uint32_t o0, uint32_t o2
 #pragma unroll 1
     for (int x = -1; x <= 1; x++) {
       LotDesc l = loadLot(W, tableSlot(o0, o2, cx + x, cz + z));
-      if (l.type >= 3 || l.h <= p.y) continue;  // (a mass below the point occludes nothing)
+      // (a mass that ends below the point, and not 1 m below the ground, occludes nothing)
+      if (l.type >= 3 || (l.h <= p.y && l.h > -1.0f)) continue;
       f3 q = toLot(p - mk(float(cx + x) * kCell + l.ox, 0.0f, float(cz + z) * kCell + l.oz), l.turn);
       float xx = fmaxf(0.0f, fabsf(q.x) - l.w), zz = fmaxf(0.0f, fabsf(q.z) - l.d);
       float dist = sqrtf(xx * xx + zz * zz);

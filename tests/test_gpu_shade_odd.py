@@ -1,6 +1,6 @@
 """Shading where its shortcuts must not be taken, against the oracle: hits at an
 infinite distance, whose noise is no number (so is the colour, unless fog covers it
-or the material has no noise)."""
+or the material has no noise), and a table with masses below the ground."""
 import numpy as np
 import pytest
 import torch
@@ -53,3 +53,14 @@ def test_hits_that_are_not_finite(cuda, oracle, t):
     assert (no_number & hits).sum() > 1000
     for got in (dropin, batched):
         assert np.array_equal(np.isnan(got), np.isnan(want))
+
+
+def test_masses_below_the_ground(cuda, oracle):
+    with ol.device_angles(oracle):
+        v, o = setup(oracle, (17.0, 2.0, 0.0), 0.0)
+        rows = o.World.reshape(-1, 16)
+        rows[np.random.default_rng(2).integers(0, 16384, 8000), 2] = -40.0
+        v.World.copy_(torch.from_numpy(o.World))
+        dropin, batched, want = both_ways(v, o, oracle)
+    for got in (dropin, batched):
+        assert np.abs(got - want).max() < 1e-4
