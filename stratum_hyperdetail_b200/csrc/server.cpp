@@ -629,8 +629,14 @@ stratum_server* stratum_server_create(unsigned long long budget_bytes, int max_v
     }
   }
   stratum_server* raw = S.release();
-  raw->worker = std::thread(schedule, raw);
-  for (int i = 0; i < kCopyThreads; i++) raw->copiers.emplace_back(copyFrames, raw);
+  try {  // a thread that cannot be started throws, which must not leave a C entry point
+    raw->worker = std::thread(schedule, raw);
+    raw->copiers.reserve(kCopyThreads);
+    for (int i = 0; i < kCopyThreads; i++) raw->copiers.emplace_back(copyFrames, raw);
+  } catch (...) {
+    stratum_server_destroy(raw);  // ends and joins those that were
+    return nullptr;
+  }
   return raw;
 }
 
