@@ -204,7 +204,8 @@ int stratum_groupCacheInit(unsigned* Groups, int entries, stratum_stream_t strea
  * order: 0 row-major, 1 Morton-ordered 4x4-tile super-tiles).  Bit 1 of order
  * selects the block-pooled trace, in which the warps of a block serve one
  * another's groups (same results; slower on the benchmark views, so
- * stratum_autotune never chooses it).  Chosen by stratum_autotune. */
+ * stratum_autotune never chooses it; calls of more than 4,095 views take the
+ * other trace).  Chosen by stratum_autotune. */
 typedef struct stratum_tune {
   int threads;
   int grab;

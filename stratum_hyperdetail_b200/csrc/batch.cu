@@ -34,7 +34,6 @@
 #include "common_api.cuh"
 #include "hierarchy.cuh"
 #include "traverse_coop.cuh"
-#include "traverse_pool.cuh"
 #include "world.cuh"
 
 static_assert(sizeof(stratum_view) == 128, "stratum_view layout is part of the ABI");
@@ -142,16 +141,6 @@ __global__ void prologueK(stratum_view* V, int n, int order, int bandTiles, Batc
   }
 }
 
-// Last view whose first tile is <= tile (binary search; warp-uniform).
-SD int viewOf(const stratum_view* __restrict__ V, int n, int tile) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (V[mid].tileBase <= tile) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 SD int bandViewOf(const BatchScratch* S, int n, int tile) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {
@@ -159,21 +148,6 @@ SD int bandViewOf(const BatchScratch* S, int n, int tile) {
     if (S->view[mid].band.base <= tile) lo = mid; else hi = mid - 1;
   }
   return lo;
-}
-
-// Claim `grab` tiles for this warp; returns the first, or >= total when empty.
-SD int claim(uint32_t* next, int grab) {
-  int t0 = 0;
-  if ((threadIdx.x & 31) == 0) t0 = int(atomicAdd(next, uint32_t(grab)));
-  return __shfl_sync(0xffffffffu, t0, 0);
-}
-// The last warp to see the queue empty resets it for the next launch.
-SD void retire(uint32_t* next, uint32_t* done, int threads) {
-  if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    uint32_t warps = gridDim.x * uint32_t(threads / 32);
-    if (atomicAdd(done, 1u) == warps - 1) { *next = 0u; *done = 0u; }
-  }
 }
 
 // STRATUM_TRACE_OCC / THREADS resident blocks (rounded down).  At 576 threads per SM
@@ -226,45 +200,6 @@ __global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
       if (!inFrame) continue;
       storeTrace(V[v].Hit, V[v].Surface, size_t(y) * W + x, r);
     }
-  }
-  retire(&S->counters[kTraceNext], &S->counters[kTraceDone], THREADS);
-}
-
-// The block-pooled trace (traverse_pool.cuh): a block claims THREADS / 32
-// tiles at once, one per warp, and its warps serve one another's groups.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, STRATUM_TRACE_OCC / THREADS)
-    tracePooledK(const stratum_view* __restrict__ V, int n, int order, BatchScratch* S) {
-  constexpr int P = THREADS / 32;
-  extern __shared__ __align__(16) unsigned char poolBytes[];
-  PoolShared<P>& sh = *reinterpret_cast<PoolShared<P>*>(poolBytes);
-  __shared__ int firstTile;
-  const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-  const int total = int(S->counters[kTotalTiles]);
-#pragma unroll 1
-  for (;;) {
-    if (threadIdx.x == 0) firstTile = int(atomicAdd(&S->counters[kTraceNext], uint32_t(P)));
-    __syncthreads();
-    const int t0 = firstTile;
-    __syncthreads();  // every thread has read it before it is written again
-    if (t0 >= total) break;
-    const int tile = t0 + warp;
-    int v = 0, W = 1, H = 1, tx = 0, ty = 0;
-    bool ok = tile < total;
-    if (ok) {
-      v = viewOf(V, n, tile);
-      W = V[v].width;
-      H = V[v].height;
-      ok = tileCoord(tile - V[v].tileBase, V[v].tilesX, (H + kTileH - 1) / kTileH, order, tx, ty);
-    }
-    const int x = tx * kTileW + (lane & 7), y = ty * kTileH + (lane >> 3);
-    const bool inFrame = ok && x < W && y < H;
-    const Camera cam = S->view[v].frame.cam;
-    const uint32_t o0 = S->view[v].frame.o[0], o2 = S->view[v].frame.o[2];
-    const f3 rd = primaryDir<Quotient>(cam, inFrame ? x : 0, inFrame ? y : 0, W, H);
-    const TraceResult r = tracePooled<P>(sh, V, v, V[v].World, reinterpret_cast<const float4*>(V[v].Nodes), o0, o2,
-                                         cam.pos, rd, 1.08f / float(H), inFrame);
-    if (inFrame) storeTrace(V[v].Hit, V[v].Surface, size_t(y) * W + x, r);
   }
   retire(&S->counters[kTraceNext], &S->counters[kTraceDone], THREADS);
 }
@@ -385,15 +320,6 @@ __global__ void __launch_bounds__(THREADS, STRATUM_RESOLVE_OCC / THREADS) resolv
   retire(&S->counters[kResolveNext], &S->counters[kResolveDone], THREADS);
 }
 
-template <class K>
-int residentBlocks(K kernel, int threads, size_t smem = 0) {
-  int dev = 0, sms = 148, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-  return sms * (per > 0 ? per : 1);
-}
 // Dynamic shared memory of a trace block: one WarpStage per warp.
 constexpr size_t traceSmem(int threads) { return size_t(threads / 32) * sizeof(WarpStage); }
 
@@ -403,8 +329,7 @@ enum Parts { kTrace = 1, kShade = 2 };
 // each kernel, computed once per (block size, device) and published through
 // std::call_once, so concurrent first calls (the render server's scheduler and
 // a direct caller) all see the four grids complete.
-constexpr int kGridDevices = 64;
-struct PersistentGrids { int trace, pooled, shade, light, resolve; };
+struct PersistentGrids { int trace, shade, light, resolve; };
 
 template <int T>
 int launchParts(stratum_view* V, int n, const stratum_tune& t, BatchScratch* S, cudaStream_t s, int parts) {
@@ -417,7 +342,6 @@ int launchParts(stratum_view* V, int n, const stratum_tune& t, BatchScratch* S, 
   std::call_once(once[dev], [&] {
     PersistentGrids g;
     g.trace = residentBlocks(traceViewsK<T>, T, traceSmem(T));
-    g.pooled = residentBlocks(tracePooledK<T>, T, sizeof(PoolShared<T / 32>));
     g.shade = residentBlocks(shadeViewsK<T>, T);
     g.light = residentBlocks(lightViewsK<T>, T);
     g.resolve = residentBlocks(resolveViewsK<T>, T);
@@ -429,8 +353,8 @@ int launchParts(stratum_view* V, int n, const stratum_tune& t, BatchScratch* S, 
     prologueK<<<1, 256, 0, s>>>(V, n, order, 2 * g.trace * (T / 32), S);
     cacheResetK<<<dim3(64, n), 256, 0, s>>>(V, n);
   }
-  if ((parts & kTrace) && (t.order & 2))
-    tracePooledK<T><<<g.pooled, T, sizeof(PoolShared<T / 32>), s>>>(V, n, order, S);
+  if ((parts & kTrace) && (t.order & 2) && n <= kPoolViews)
+    launchPooled<T>(V, n, order, S, dev, s);
   else if (parts & kTrace)
     traceViewsK<T><<<g.trace, T, traceSmem(T), s>>>(V, n, t.grab, order, S);
   if (parts & kShade) shadeViewsK<T><<<g.shade, T, 0, s>>>(V, n, t.grab, order, S);

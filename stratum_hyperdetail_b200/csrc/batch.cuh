@@ -85,4 +85,45 @@ SD int bandCount(const Band& b, int tilesX, int height) {
   return (min(b.row1 * kTileH, height) - b.row0 * kTileH) * tilesX;
 }
 
+// Last view whose first tile is <= tile (binary search; warp-uniform).
+SD int viewOf(const stratum_view* __restrict__ V, int n, int tile) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (V[mid].tileBase <= tile) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Claim `grab` tiles for this warp; returns the first, or >= total when empty.
+SD int claim(uint32_t* next, int grab) {
+  int t0 = 0;
+  if ((threadIdx.x & 31) == 0) t0 = int(atomicAdd(next, uint32_t(grab)));
+  return __shfl_sync(0xffffffffu, t0, 0);
+}
+// The last warp to see the queue empty resets it for the next launch.
+SD void retire(uint32_t* next, uint32_t* done, int threads) {
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    uint32_t warps = gridDim.x * uint32_t(threads / 32);
+    if (atomicAdd(done, 1u) == warps - 1) { *next = 0u; *done = 0u; }
+  }
+}
+
+// Blocks of a kernel that the current device holds.
+template <class K>
+inline int residentBlocks(K kernel, int threads, size_t smem = 0) {
+  int dev = 0, sms = 148, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
+  return sms * (per > 0 ? per : 1);
+}
+
+// The block-pooled trace of at most kPoolViews views, with the device's ordinal (pooled.cu).
+constexpr int kPoolViews = 4095, kGridDevices = 64;
+template <int THREADS>
+void launchPooled(const stratum_view* V, int n, int order, BatchScratch* S, int dev, cudaStream_t stream);
+
 }  // namespace st

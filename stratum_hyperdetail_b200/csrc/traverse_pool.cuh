@@ -15,6 +15,7 @@
 // (__syncthreads_or), so all threads of the block, rays in flight or not, reach
 // the same barriers.
 #pragma once
+#include "batch.cuh"
 #include "traverse_coop.cuh"
 
 namespace st {
@@ -29,19 +30,20 @@ struct PoolShared {
   PoolStage stage[P];
   float lr[3][P * 32], ld[3][P * 32], inv[3][P * 32];
   float best[P * 32], cone[P * 32];
-  unsigned long long key[P * 32];  // pending head (poolKey), or kPoolIdle
-  int fid[P * 32];                 // winner (group * 64 + index) after a serve that improved best
+  unsigned key[P * 32];  // pending head (poolKey), or kPoolIdle
+  int fid[P * 32];       // winner (group * 64 + index) after a serve that improved best
 };
 
-// A head of any view a launch takes (65,535: 36 bits).
-constexpr unsigned long long kPoolIdle = ~0ull;
-HD unsigned long long poolKey(int view, int slot, int group) {
-  return (unsigned long long)view << 20 | unsigned(slot << 6 | group);
-}
-HD int poolView(unsigned long long key) { return int(key >> 20); }
-HD int poolGroupKey(unsigned long long key) { return int(key & 0xFFFFFu); }  // slot << 6 | group
+// Heads name kPoolViews views (12 bits; the last value is an idle lane's).  64-bit heads
+// would name all that a launch takes, but cost 128-thread blocks 5-9 % (spills); calls of
+// more views take the per-warp trace.
+constexpr unsigned kPoolIdle = ~0u;
+static_assert(kPoolViews < 1 << 12, "a head has 12 bits for its view");
+HD unsigned poolKey(int view, int slot, int group) { return unsigned(view) << 20 | unsigned(slot << 6 | group); }
+HD int poolView(unsigned key) { return int(key >> 20); }
+HD int poolGroupKey(unsigned key) { return int(key & 0xFFFFFu); }  // slot << 6 | group
 template <int P>
-SD int poolWarpOf(unsigned long long key) { return int((unsigned(key) * 2654435761u) >> 16) % P; }
+SD int poolWarpOf(unsigned key) { return int((key * 2654435761u) >> 16) % P; }
 
 // One ray of the block against the group staged in `ws` (the record loop of
 // traceWarp, on the ray's state in shared memory).
@@ -86,7 +88,7 @@ SD void poolTest(PoolShared<P>& sh, int j, const PoolStage& ws, int count, int g
 template <int P>
 SD void poolServe(PoolShared<P>& sh, const stratum_view* __restrict__ V) {
   const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-  unsigned long long kk[P];
+  unsigned kk[P];
   unsigned mine[P];
 #pragma unroll
   for (int p = 0; p < P; p++) {
@@ -95,7 +97,7 @@ SD void poolServe(PoolShared<P>& sh, const stratum_view* __restrict__ V) {
   }
 #pragma unroll 1
   for (;;) {
-    unsigned long long key = kPoolIdle;
+    unsigned key = kPoolIdle;
 #pragma unroll
     for (int p = 0; p < P; p++)
       if (key == kPoolIdle && mine[p]) key = __shfl_sync(0xffffffffu, kk[p], __ffs(mine[p]) - 1);

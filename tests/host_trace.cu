@@ -39,7 +39,7 @@ extern "C" int ht_heads(const int* heads, int n) {
   int good = 0;
   for (int i = 0; i < n; i++) {
     const int v = heads[3 * i], slot = heads[3 * i + 1], g = heads[3 * i + 2];
-    const unsigned long long k = poolKey(v, slot, g);
+    const unsigned k = poolKey(v, slot, g);
     good += k != kPoolIdle && poolView(k) == v && poolGroupKey(k) == (slot << 6 | g);
   }
   return good;
