@@ -6,9 +6,8 @@
 // five launches (prepare, forward, score, gradient, Adam) are one block here:
 // the samples' work rows and the gradient stay in shared memory and the phases
 // are separated by block barriers.
-#include "common_api.cuh"
-#include "frame_init.cuh"
 #include "neural.cuh"
+#include "strips.cuh"
 
 namespace st {
 
@@ -190,12 +189,17 @@ __global__ void predictSubstrateK(const float* __restrict__ W, const float* __re
   Out[size_t(i) * 3] = c.x; Out[size_t(i) * 3 + 1] = c.y; Out[size_t(i) * 3 + 2] = c.z;
 }
 
-// The material half of shadePixels with the surrogate in place of the procedural
-// substrate of brick and stone when C[16] enables it and the gate Brain[4] is open
-// (Stratum.cu:854); otherwise exactly the drop-in's.  The lighting half follows as
-// its own kernel (shade.cu).
-constexpr int kNeuralThreads = 128;
-__global__ void __launch_bounds__(kNeuralThreads, 1024 / kNeuralThreads)
+// The albedo of a hit pixel with the surrogate in place of the procedural substrate of
+// brick and stone when `useNet` (Stratum.cu:854); otherwise exactly the drop-in's.
+SD f3 neuralAlbedo(const float* __restrict__ W, const SurfacePoint& sp, bool useNet) {
+  f3 base = substrateMean(sp.mat);
+  if (sp.mat == 0 || sp.mat == 1)
+    base = useNet ? predictSubstrate(W, sp.u, sp.v, sp.seed, sp.mat) : substrate(sp.u, sp.v, sp.seed, sp.mat);
+  return surfaceColor(sp.q, sp.qn, sp.mat, sp.seed, sp.sfp, base) * paletteTint(sp.palette, sp.mat);
+}
+// The material half of shadePixels with the surrogate, when C[16] enables it and the
+// gate Brain[4] is open.  The lighting half follows as its own kernel (shade.cu).
+__global__ void __launch_bounds__(kShadeThreads, 1024 / kShadeThreads)
     albedoNeuralK(const float* __restrict__ World, const uint32_t* __restrict__ O, const float* __restrict__ C,
                   const float4* __restrict__ Hit, const float4* __restrict__ Surface, float4* Linear,
                   const float* __restrict__ W, const float* __restrict__ Brain, int width, int height, int rowStart,
@@ -203,12 +207,11 @@ __global__ void __launch_bounds__(kNeuralThreads, 1024 / kNeuralThreads)
   __shared__ FrameConst F;
   frameInit(F, C, O);
   const bool useNet = C[16] > 0.5f && Brain[4] > 0.5f;
-  const int tilesX = (width + 7) / 8, tiles = tilesX * ((rowEnd - rowStart + 3) / 4), warps = kNeuralThreads / 32;
-  const int lane = int(threadIdx.x & 31);
+  const int tilesX = (width + 7) / 8, tiles = tilesX * ((rowEnd - rowStart + 3) / 4), warps = kShadeThreads / 32;
 #pragma unroll 1
   for (int i = int(blockIdx.x) * warps + int(threadIdx.x >> 5); i < tiles; i += int(gridDim.x) * warps) {
-    const int x = (i % tilesX) * 8 + (lane & 7), y = rowStart + (i / tilesX) * 4 + (lane >> 3);
-    if (x >= width || y >= rowEnd) continue;
+    int x, y;
+    if (!stripPixel(i, tilesX, width, rowStart, rowEnd, x, y)) continue;
     const size_t b = size_t(y) * width + x;
     const f3 rd = primaryDir(F.cam, x, y, width, height);
     const float4 h = Hit[b];
@@ -218,13 +221,35 @@ __global__ void __launch_bounds__(kNeuralThreads, 1024 / kNeuralThreads)
     } else {
       SurfacePoint sp;
       surfacePoint(World, F, h, Surface[b], rd, height, sp);
-      f3 base = substrateMean(sp.mat);
-      if (sp.mat == 0 || sp.mat == 1)
-        base = useNet ? predictSubstrate(W, sp.u, sp.v, sp.seed, sp.mat) : substrate(sp.u, sp.v, sp.seed, sp.mat);
-      c = surfaceColor(sp.q, sp.qn, sp.mat, sp.seed, sp.sfp, base) * paletteTint(sp.palette, sp.mat);
+      c = neuralAlbedo(W, sp, useNet);
     }
     Linear[b] = make_float4(c.x, c.y, c.z, 1.0f);
   }
+}
+// Both halves at once, for strips of at most one wave (strips.cuh).
+__global__ void __launch_bounds__(kShadeThreads, 1024 / kShadeThreads)
+    shadePixelsNeuralK(const float* __restrict__ World, const uint32_t* __restrict__ O, const float* __restrict__ C,
+                       const float4* __restrict__ Hit, const float4* __restrict__ Surface, float4* Linear,
+                       const float* __restrict__ W, const float* __restrict__ Brain, int width, int height, int rowStart,
+                       int rowEnd) {
+  __shared__ FrameConst F;
+  frameInit(F, C, O);
+  int x, y;
+  if (!stripPixel(int(blockIdx.x) * (kShadeThreads / 32) + int(threadIdx.x >> 5), (width + 7) / 8, width, rowStart, rowEnd,
+                  x, y))
+    return;
+  const size_t b = size_t(y) * width + x;
+  const f3 rd = primaryDir(F.cam, x, y, width, height);
+  const float4 h = Hit[b];
+  f3 c;
+  if (int(h.y) == kSkyId) {
+    c = skyColor(rd, F.sun);
+  } else {
+    SurfacePoint sp;
+    surfacePoint(World, F, h, Surface[b], rd, height, sp);
+    c = pixelLight(World, F, sp, rd, int(h.y), neuralAlbedo(W, sp, C[16] > 0.5f && Brain[4] > 0.5f));
+  }
+  Linear[b] = make_float4(c.x, c.y, c.z, 1.0f);
 }
 
 // The lighting half of shadePixels (shade.cu).
@@ -268,8 +293,15 @@ int stratum_shadePixelsNeural(const float* World, const unsigned* Origin, const 
   if (rowStart < 0 || rowCount < 0) return STRATUM_EINVAL;
   const int rows = rowCount < height - rowStart ? rowCount : height - rowStart;
   if (rows <= 0) return STRATUM_OK;
-  const int need = ((width + 7) / 8 * ((rows + 3) / 4) + 3) / 4, most = 148 * (1024 / kNeuralThreads);
-  albedoNeuralK<<<need < most ? need : most, kNeuralThreads, 0, asStream(stream)>>>(
+  const int wave = shadeWave();
+  if (!wave) return STRATUM_EINVAL;
+  if (tileBlocks(width, rows) <= wave) {
+    shadePixelsNeuralK<<<tileBlocks(width, rows), kShadeThreads, 0, asStream(stream)>>>(
+        World, Origin, C, reinterpret_cast<const float4*>(Hit), reinterpret_cast<const float4*>(Surface),
+        reinterpret_cast<float4*>(Linear), W, Brain, width, height, rowStart, rowStart + rows);
+    return launchStatus();
+  }
+  albedoNeuralK<<<tileBlocks(width, rows, wave), kShadeThreads, 0, asStream(stream)>>>(
       World, Origin, C, reinterpret_cast<const float4*>(Hit), reinterpret_cast<const float4*>(Surface),
       reinterpret_cast<float4*>(Linear), W, Brain, width, height, rowStart, rowStart + rows);
   const int s = launchStatus();

@@ -5,26 +5,16 @@
 // block works out the frame's constants once, an angle a lane: with 64-pixel
 // blocks of a wave each, every block waited for one thread's eight double sines.
 // Material and light are two kernels, as in the batched path (albedo into Linear,
-// then lit in place): half the code for the instruction cache.  One 1600x900 frame
+// then lit in place): half the code for the instruction cache; short strips are shaded by
+// one (strips.cuh).  One 1600x900 frame
 // (mean of six poses): shade 275 us in one kernel of 8x8 blocks, now 220 us; resolve
 // 118 us, now 89 us.
 #include <mutex>
 
-#include "common_api.cuh"
-#include "frame_init.cuh"
 #include "shading.cuh"
+#include "strips.cuh"
 
 namespace st {
-
-constexpr int kShadeThreads = 128;
-
-// Tile `i` of a strip of rows: whether this lane has a pixel there, and which.
-SD bool stripPixel(int i, int tilesX, int width, int rowStart, int rowEnd, int& x, int& y) {
-  const int lane = int(threadIdx.x & 31);
-  x = (i % tilesX) * 8 + (lane & 7);
-  y = rowStart + (i / tilesX) * 4 + (lane >> 3);
-  return x < width && y < rowEnd;
-}
 
 __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads)
     albedoPixelsK(const float* __restrict__ W, const uint32_t* __restrict__ O, const float* __restrict__ C,
@@ -75,6 +65,31 @@ __global__ void __launch_bounds__(kShadeThreads, 1536 / kShadeThreads)
   }
 }
 
+// Both halves at once, for strips of at most one wave (strips.cuh).
+__global__ void __launch_bounds__(kShadeThreads, 1024 / kShadeThreads)
+    shadePixelsK(const float* __restrict__ W, const uint32_t* __restrict__ O, const float* __restrict__ C,
+                 const float4* __restrict__ Hit, const float4* __restrict__ Surface, float4* Linear, int width,
+                 int height, int rowStart, int rowEnd) {
+  __shared__ FrameConst F;
+  frameInit(F, C, O);
+  int x, y;
+  if (!stripPixel(int(blockIdx.x) * (kShadeThreads / 32) + int(threadIdx.x >> 5), (width + 7) / 8, width, rowStart, rowEnd,
+                  x, y))
+    return;
+  const size_t b = size_t(y) * width + x;
+  const float4 h = Hit[b];
+  const f3 rd = primaryDir(F.cam, x, y, width, height);
+  f3 c;
+  if (int(h.y) == kSkyId) {
+    c = skyColor(rd, F.sun);
+  } else {
+    SurfacePoint sp;
+    surfacePoint(W, F, h, Surface[b], rd, height, sp);
+    c = pixelLight(W, F, sp, rd, int(h.y), pixelAlbedo(sp));
+  }
+  Linear[b] = make_float4(c.x, c.y, c.z, 1.0f);
+}
+
 __global__ void __launch_bounds__(kShadeThreads, 1024 / kShadeThreads)
     resolveFrameK(const float4* __restrict__ Linear, float4* History, uint32_t* Pixels, const float* __restrict__ C,
                   const float4* __restrict__ Hit, const float4* __restrict__ Surface, int width, int height) {
@@ -112,11 +127,6 @@ const ShadeGrids* shadeGrids() {
   });
   return &grids[dev];
 }
-int tileBlocks(int width, int rows, int held) {
-  const int need = ((width + 7) / 8 * ((rows + 3) / 4) + kShadeThreads / 32 - 1) / (kShadeThreads / 32);
-  return need < held ? need : held;
-}
-
 // The lighting half alone, over an albedo that is already in Linear.
 int lightRows(const float* World, const unsigned* Origin, const float* C, const float* Hit, const float* Surface,
               float* Linear, int width, int height, int rowStart, int rows, cudaStream_t stream) {
@@ -143,6 +153,12 @@ int stratum_shadePixels(const float* World, const unsigned* Origin, const float*
   if (rows <= 0) return STRATUM_OK;
   const ShadeGrids* g = shadeGrids();
   if (!g) return STRATUM_EINVAL;
+  if (tileBlocks(width, rows) <= shadeWave()) {
+    shadePixelsK<<<tileBlocks(width, rows), kShadeThreads, 0, asStream(stream)>>>(
+        World, Origin, C, reinterpret_cast<const float4*>(Hit), reinterpret_cast<const float4*>(Surface),
+        reinterpret_cast<float4*>(Linear), width, height, rowStart, rowStart + rows);
+    return launchStatus();
+  }
   albedoPixelsK<<<tileBlocks(width, rows, g->albedo), kShadeThreads, 0, asStream(stream)>>>(
       World, Origin, C, reinterpret_cast<const float4*>(Hit), reinterpret_cast<const float4*>(Surface),
       reinterpret_cast<float4*>(Linear), width, height, rowStart, rowStart + rows);

@@ -20,6 +20,13 @@ def _s(stream):
     return (stream or torch.cuda.current_stream()).cuda_stream
 
 
+def shade_launches(width: int, rows: int, device) -> int:
+    """Kernels that stratum_shadePixels launches for a strip: one up to 32 tiles of 8x4
+    pixels an SM, else material, then light."""
+    tiles = (width + 7) // 8 * ((rows + 3) // 4)
+    return 1 if tiles <= 32 * torch.cuda.get_device_properties(device).multi_processor_count else 2
+
+
 class View:
     def __init__(self, width: int, height: int, device="cuda"):
         self.width, self.height = int(width), int(height)
@@ -111,7 +118,7 @@ class View:
         for y in range(0, h, ROWS):
             call("stratum_shadePixels", ptr(self.World), ptr(self.Origin), ptr(self.C), ptr(self.Hit), ptr(self.Surface),
                  ptr(self.Linear), w, h, y, min(ROWS, h - y), s)
-            n += 2  # material, then light
+            n += shade_launches(w, min(ROWS, h - y), self.World.device)
         call("stratum_resolveFrame", ptr(self.Linear), ptr(self.History), ptr(self.Pixels), ptr(self.C), ptr(self.Hit),
              ptr(self.Surface), w, h, s)
         return n + 1
