@@ -129,15 +129,20 @@ extern "C" int stratum_tracePrimary(const float* World, const float* Nodes, cons
     resident[dev] = sms * STRATUM_DROPIN_BLOCKS;
   });
   // Band rows: up to twice the blocks the device holds in quarter blocks, but at
-  // most a sixth of a frame that fills the device by itself (a band row takes about
-  // two rows' time; a 64-row strip gets none), and none in one that fills it more than
-  // 14 times, whose other rows hide the slow tiles.  One call for each of six poses, sum
-  // in us, without / with: 320x180 2,045 / 1,507, 640x360 2,454 / 2,118, 1024x576 (7.8
-  // times) 3,380 / 3,167, 1283x721 (12.6) 4,125 / 4,099, 1600x900 (19) 4,948 / 5,238,
-  // 3840x2160 18,635 / 18,970.
+  // most a sixth of a launch that fills the device by itself (a band row takes about
+  // two rows' time; so a 64-row strip that does gets none), and none in one that fills it
+  // more than 14 times, whose other rows hide the slow tiles.  One call for each of six
+  // poses, sum in us, without / with: 320x180 2,045 / 1,507, 640x360 2,454 / 2,118, 1024x576
+  // (7.8 times) 3,380 / 3,167, 1283x721 (12.6) 4,199 / 4,151, 1344x756 (13.6) 4,359 / 4,235,
+  // 1440x810 (15.5) 4,463 / 4,632, 1600x900 (19) 5,031 / 5,305, 3840x2160 18,635 / 18,970.
+  // A launch that does not fill the device may be all band: a small frame has to be, but
+  // most strips of a larger one hold no horizon, and a strip of over 0.6 of the device
+  // gets none.  Frames in 64-row strips: 320x180 (strips of 0.3 of the device) 3,115 / 2,116,
+  // 640x360 (0.5) 4,674 / 4,315, 800x450 (0.7) 5,314 / 6,321, 1024x576 (0.9) 6,146 / 8,231.
   const int blocksX = (width + kDropInW - 1) / kDropInW, blockRows = (rows + kDropInH - 1) / kDropInH;
-  const int blocks = blocksX * blockRows;
-  const int most = blocks <= resident[dev] ? blockRows : blocks <= 14 * resident[dev] ? blockRows / 6 : 0;
+  const int blocks = blocksX * blockRows, held = resident[dev];
+  const bool all = blocks <= held && (rows == height || 5 * blocks <= 3 * held);
+  const int most = all ? blockRows : blocks <= 14 * held ? blockRows / 6 : 0;
   const int want = (2 * resident[dev] - 1) / (4 * blocksX) + 1, bandRows = want < most ? want : most;
   tracePrimaryK<<<blocksX * (blockRows + 4 * bandRows), kDropInThreads, sizeof(DropInShared), asStream(stream)>>>(
       World, Nodes, static_cast<const uint32_t*>(Origin), C, Hit, Surface, width, height, rowStart, rowCount, blocksX,
