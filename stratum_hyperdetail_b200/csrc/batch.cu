@@ -154,7 +154,8 @@ SD int bandViewOf(const BatchScratch* S, int n, int tile) {
 // the compiler takes 96 registers, which is ten 64-thread blocks: six-view 1600x900
 // trace 3.45 ms, aerial 1.54; 512 (128 registers) 3.73 / 1.69, 640 3.51 / 1.57.  768
 // (80 registers, spills) is equal over whole frames, but the slowest tiles, which bound
-// small views, take 5-10 % longer.
+// small views, take 5-10 % longer.  128- and 256-thread blocks come to four and two an SM
+// (127 registers, 16 warps): 3.49 and 3.48 ms.
 #ifndef STRATUM_TRACE_OCC
 #define STRATUM_TRACE_OCC 576
 #endif

@@ -24,7 +24,8 @@
 // in every warp that meets it: first batched 1600x900 frame, street 2.17 -> 1.69 ms,
 // aerial 6.40 -> 3.90 ms, avenue 2.04 -> 1.29 ms; frames of a filled cache are
 // unchanged.  (The winner's record, once a ray, is rebuilt instead in that frame:
-// reading it too takes 0.2 ms off the aerial pose and 1 % onto every later frame.)  A warp that misses claims the group (one atomic compare-and-swap on its
+// reading it too takes 0.2 ms off the aerial pose and 1 % onto every later frame.)
+// A warp that misses claims the group (one atomic compare-and-swap on its
 // directory word) and fills an entry, or, when another warp holds it or the
 // store is full, builds the records with the grammar itself: nothing waits.
 // A full store keeps serving the groups it holds; at the start of a launch at
@@ -152,7 +153,7 @@ SD int cacheClaim(const GroupCache& c, int slot, int group, uint32_t old) {
 }
 
 // Warp-collective: publish a claimed entry whose records the lanes have
-// written.  Readers use it from the next launch on.
+// written.  Other warps of the launch may read it from then on (filledNow).
 SD void cachePublish(const GroupCache& c, const float* W, int slot, int group, int count, int e) {
   const int lane = int(threadIdx.x & 31);
   if (lane < kEntryTagWords) entryTag(c, uint32_t(e))[lane] = tagWord(W + size_t(slot) * kLotFloats, group, count, lane);

@@ -10,7 +10,7 @@
 //    next lots in turn, whatever their distance: 3.88 ms against 3.45, below).  Lanes
 //    stand for leaves: all 64 groups of the lot are tested at once against the
 //    waiting rays, taken as a packet (packetMayEnter), and each ray then tests the few
-//    leaves left (3-6) itself and orders its own by the reference's near-first descent,
+//    leaves left (3-7) itself and orders its own by the reference's near-first descent,
 //    which needs the hierarchy only where the paths to two of its leaves part;
 //  * the warp evaluates one group of that lot at a time for all the lanes that wait
 //    on it, the one whose ray has the most leaves to go first, since a ray that is
@@ -19,14 +19,14 @@
 //    from the table's group cache (group_cache.cuh), the block's table (the
 //    drop-in), or the random-access grammar (grammar_ra.cuh), which stores them
 //    when the cache has room.  Lanes now stand for records and test them against
-//    the packet (packetMayHit): most evaluations end there (63 % on the street pose,
-//    38 % on the aerial one, keep no record, the others 2-5 of up to 56), and the
+//    the packet (packetMayHit): many evaluations end there (64 % on the street pose,
+//    30 % on the aerial one, keep no record, the others 2-7 of up to 56), and the
 //    waiting lanes test the records kept, in index order, with one inlined
 //    intersection routine;
 //  * the winner's normal, material and seed are recomputed once per ray.
 //
-// What bounds the kernel is waiting for instructions (4 of the 9 cycles a warp waits
-// per issue: a tile runs once through most of its 87 KB of code), then dependent
+// What bounds the kernel is waiting for instructions (a third of a warp's waiting: a
+// tile runs once through most of its 87 KB of code), then dependent
 // arithmetic and loads.  One copy of each division, square root and of the step to
 // the next leaf took the six-view trace from 4.62 to 4.14 ms at 108 -> 87 KB; at 150 KB
 // the aerial pose took twice as long.  Lots and groups in the order above: 3.45 ms
